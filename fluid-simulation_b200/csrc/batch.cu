@@ -121,6 +121,14 @@ struct BatchSim {
         }
     }
 
+    // density units: see CUDASPHSimulator::use_units
+    bool use_units() const { return nbr_width > 0 && dp.range == 1; }
+    // The persistent kernel's 256-thread blocks take units of 4x4x2 cells at
+    // least (12 / 64 / 256 scenes, ms per step at levels 3, 5, 6: 0.571 / 1.81 /
+    // 6.80, 0.455 / 1.28 / 4.49, 0.480 / 1.27 / 4.33).
+    u32 batch_unit_level(bool persistent) const { return persistent ? std::max(unit_level(n), 5u) : unit_level(n); }
+    u32* unit_buf() { return reinterpret_cast<u32*>(keys[1].ptr); }
+
     // persistent: the persistent kernel's traversal phases (16 particles per
     // warp chunk; the per-stage passes take 32, 3 % faster on the 256-scene
     // ensemble, where 32 slows the persistent launch). Results do not depend
@@ -144,8 +152,10 @@ struct BatchSim {
         a.mask = mask.ptr;
         a.mask_words = static_cast<u32>(mask_words);
         a.chunk = n < (1u << 18) ? 8u : (persistent ? 16u : 32u);
+        a.units = use_units() ? unit_buf() : nullptr;
+        a.unit_level = batch_unit_level(persistent);
         a.nbr = nbr_width > 0 ? nbr.ptr : nullptr;
-        a.pair_cells = a.nbr != nullptr ? 1u : 0u;
+        a.keep_matrix = a.nbr == nullptr ? 1u : 0u;
         a.nbr_cnt = nbr_cnt.ptr;
         a.nbr_width = static_cast<u32>(nbr_width);
         a.rho = rho.ptr; a.prs = prs.ptr;
@@ -178,7 +188,7 @@ struct BatchSim {
         WCSPH_CUDA(enqueue_sort_passes(sb, n, st.ptr, stream));
         launch_reorder_cells(pos_a.ptr, vel_a.ptr, vals[1].ptr, vals[2].ptr, st.ptr, n, dp.cell_size, pos_b.ptr,
                              vel_b.ptr, perm.ptr, ckey.ptr, table.ptr, cstart.ptr, cend.ptr, table_size - 1, st.ptr,
-                             stream, scene_a.ptr);
+                             stream, scene_a.ptr, use_units() ? unit_buf() : nullptr, batch_unit_level(false));
         const TravArgs a = args(delta);
         launch_pass(PASS_DENSITY, dp, a, stream, 2, true);
         launch_pass(PASS_FORCE, dp, a, stream, 2, true);

@@ -77,13 +77,18 @@ __device__ __forceinline__ bool grid_barrier(u32* bar, DevState* st, u32 limit) 
     return s_go != 0u;
 }
 
+// Density units in the persistent kernel: 256-thread blocks, the largest capacity.
+struct PersistentBlock {
+    static constexpr int nt = PTHREADS, cap = 3072, words = 12;
+};
+
 size_t persistent_smem(const TravArgs& a) {
     const u32 cap = a.mask_words * 32u;
     const u32 ncell = static_cast<u32>((2 * a.range + 1) * (2 * a.range + 1) * (2 * a.range + 1));
     const bool wb = a.nb > 0;
     size_t b = sizeof(u32) * SORT_DIGITS * 256;                  // digit histograms
     b = std::max(b, sizeof(u32) * (PWARPS * 256 + 256));          // onesweep ranks and bases
-    b = std::max(b, PWARPS * warp_smem_bytes<PASS_DENSITY>(cap, ncell, wb));
+    b = std::max(b, a.units ? sizeof(BlockSmem<PersistentBlock>) : PWARPS * warp_smem_bytes<PASS_DENSITY>(cap, ncell, wb));
     if (a.nbr == nullptr) {                                       // force and surface walk the bit matrix
         b = std::max(b, PWARPS * warp_smem_bytes<PASS_FORCE>(cap, ncell, wb));
         b = std::max(b, PWARPS * warp_smem_bytes<PASS_SURFACE>(cap, ncell, wb));
@@ -139,10 +144,13 @@ __global__ void __launch_bounds__(PTHREADS, 3) persistent_ensemble_kernel(const 
             reorder_cell_item<true>(ps.pos_state, ps.vel_state, ps.vals[1], ps.vals[2], st, n, ps.cs,
                                     const_cast<float4*>(a.pos), const_cast<float4*>(a.vel), ps.perm,
                                     const_cast<u64*>(a.ckey), ps.table, const_cast<u32*>(a.fluid.cstart),
-                                    const_cast<u32*>(a.fluid.cend), a.fluid.tmask, st, ps.scene_state, base + tid);
+                                    const_cast<u32*>(a.fluid.cend), a.fluid.tmask, st, ps.scene_state, base + tid,
+                                    const_cast<u32*>(a.units), a.unit_level);
         if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;
         const u32 nchunks = (n + a.chunk - 1) / a.chunk;
-        {
+        if (a.units) {
+            density_units<PersistentBlock, true>(P, a, *reinterpret_cast<BlockSmem<PersistentBlock>*>(smem));
+        } else {
             const WarpView<PASS_DENSITY> S = warp_view<PASS_DENSITY>(a, smem, warp);
             for (u32 c0 = claim(ps.barrier + WORK_DENSITY); c0 < nchunks; c0 = claim(ps.barrier + WORK_DENSITY))
                 for (u32 c = c0; c < min(c0 + CLAIM, nchunks); ++c)

@@ -1,0 +1,394 @@
+// density_blocks.cuh — the density pass over blocks of cells (one neighbour
+// cell in every direction, neighbour lists on).
+//
+// A unit of work is a Morton-aligned block of cells (2x2x2, 4x4x2 or 4x4x4:
+// its particles are contiguous in sorted order) and one thread block of NT
+// threads. The unit
+//   1. counts its particles (rows) and looks up the cells of the block and of
+//      the layer around it (64, 144 or 216), one thread per cell;
+//   2. stages their particles (the candidates) in shared memory, cells in the
+//      x, y, z nesting order, as x / y / z / particle-index arrays;
+//   3. lets every lane take one row. The 27 cells around the row's cell are 9
+//      runs of 3 cells that lie next to each other in the staged order, so
+//      the row's candidates are 9 segments, in the reference's order. The lane
+//      tests a segment four candidates at a time (three 128-bit shared loads,
+//      packed FP32 in the rounding of dist2) and shifts the results into a
+//      32-bit word: r2 <= h2 holds exactly when r2 - (the float after h2) is
+//      negative, so a funnel shift collects the sign bits, without compares.
+//      Words with hits are kept in shared memory (one column per thread), then
+//      the lane walks their bits: it sums W and writes its list, slot t of
+//      all lanes of a warp in one 128-byte store.
+// Rows hold 25 to 45 neighbours, so the lanes of a warp finish together
+// within a few hits, and no partial sums cross lanes: a row's sum runs over its
+// neighbours in the reference's order whatever the block size.
+//
+// What bounds it (1 M particles, 4x4x4 cells): instruction issue (141 M warp
+// instructions, 61 % of the cycles issue) and the shared-memory data pipe
+// (75 % busy: a 128-bit load costs three wavefronts for a warp's four or five
+// cells, a walked hit four loads of four). Of its 208 us, look-ups and counts
+// take about 35 (latency), staging 18, the tests 85, the walk 61, the epilogue
+// 18. The pass it replaced gave a warp the two cells of an x-pair (36 looked-up
+// cells and 18 staged candidates per row, where a row here pays for 3.4), split
+// their hits over the lanes and wrote the lists one scattered word at a time:
+// 349 M warp instructions, 460 us (4 M particles 2055 -> 823 us, 0.7 M settled
+// 434 -> 251, 33 k with walls 51 -> 30).
+#pragma once
+
+namespace wcsph {
+namespace {
+
+// Threads per unit, candidate capacity and hit words per row. The capacity is
+// 12 to 16 particles per cell (the 0.92-spaced, settled fluid holds 10.3);
+// denser blocks are split into smaller ones. The thread counts fit the rows of
+// a block into whole rounds: 4x4x4 cells hold 512 rows and a few (17 groups of
+// 32), two rounds of 9 warps and three of 8 (4 M particles: 853 us against 930).
+template <int LEVEL>
+struct BlockCfg;
+template <>
+struct BlockCfg<3> {   // 2x2x2 cells
+    static constexpr int nt = 96, cap = 1024, words = 12, min_blocks = 8;
+};
+template <>
+struct BlockCfg<5> {   // 4x4x2 cells
+    static constexpr int nt = 256, cap = 2048, words = 12, min_blocks = 4;
+};
+template <>
+struct BlockCfg<6> {   // 4x4x4 cells
+    static constexpr int nt = 288, cap = 2560, words = 12, min_blocks = 3;
+};
+
+constexpr int BLOCK_CELLS = 216;   // cells of the largest block with its surrounding layer
+
+template <class C>
+struct BlockSmem {
+    float x[C::cap], y[C::cap], z[C::cap];
+    u32 j[C::cap];
+    u32 word[C::words * C::nt];
+    unsigned short wbase[C::words * C::nt];
+    u32 rstart[BLOCK_CELLS];
+    u32 rpref[BLOCK_CELLS + 4];
+    u32 next;   // the unit claimed next
+};
+
+// Density of row i's boundary particles (cell size h cells, one lane): its
+// cell's candidate run, tested 32 at a time, then the hits in run order. The
+// first 128 results are the row's hit mask for the force pass.
+template <bool BATCH>
+__device__ __forceinline__ void density_boundary_row(const DevParams& P, const TravArgs& a, float4 xi, u32 scene,
+                                                     u32 i, float* resb) {
+    HomeData H;
+    H.x = xi;
+    if (a.bcell.table == nullptr) {
+        boundary_row<PASS_DENSITY, BATCH>(P, a, H, scene, resb, i);
+        return;
+    }
+    u32 t, e;
+    boundary_run<BATCH>(a, boundary_cell_key<BATCH>(cell_of(xi, P.h), scene), t, e);
+    u32 mk[4] = {0u, 0u, 0u, 0u};
+    for (u32 w = 0; t + 32u * w < e; ++w) {
+        const u32 b0 = t + 32u * w;
+        const u32 len = min(32u, e - b0);
+        u32 bits = 0;
+#pragma unroll 4
+        for (u32 u = 0; u < len; ++u) {
+            const float4 xb = ro_ld(a.bcx + guard(a, b0 + u, a.bcx_n));
+            bits |= (dist2(xi, xb) <= P.h2 ? 1u : 0u) << u;
+        }
+#pragma unroll
+        for (u32 q = 0; q < 4; ++q)
+            if (w == q) mk[q] = bits;
+        for (; bits; bits &= bits - 1) {
+            const float4 xb = ro_ld(a.bcx + guard(a, b0 + (__ffs(bits) - 1), a.bcx_n));
+            boundary_pair_m<PASS_DENSITY>(resb, H, xb.w, xb, dist2(xi, xb), P);
+        }
+    }
+    if (a.bmask != nullptr) a.bmask[i] = make_uint4(mk[0], mk[1], mk[2], mk[3]);
+}
+
+// Sum of W of one pair: 2 (1 - q)^3 - max(1 - 2 q, 0)^3 is the cubic spline
+// over its factor for q <= 1; the two cubes are summed apart. The rounding is
+// written out: every kernel that inlines this produces the same bits.
+__device__ __forceinline__ void density_pair(float r2, const DevParams& P, float& t3, float& u3) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(r2));
+    const float q = __fmul_rn(r, P.inv_h);
+    const float t = __fsub_rn(1.f, q);
+    const float u = fmaxf(__fmaf_rn(-2.f, q, 1.f), 0.f);
+    t3 = __fmaf_rn(__fmul_rn(t, t), t, t3);
+    u3 = __fmaf_rn(__fmul_rn(u, u), u, u3);
+}
+
+// Row i without staged candidates (a single cell whose 27 cells exceed the
+// capacity): its cells one after the other from global memory, in the same
+// order. Returns the neighbour count.
+template <bool BATCH>
+__device__ __forceinline__ u32 density_direct_row(const DevParams& P, const TravArgs& a, u32 i, u64 pk, float4 xi,
+                                                  float& t3, float& u3) {
+    u32 ux, uy, uz, scene;
+    decode_cell<BATCH>(pk, ux, uy, uz, scene);
+    u32 hits = 0;
+    for (u32 q = 0; q < 27u; ++q) {
+        int dx, dy, dz;
+        cell_offset(q, 1, dx, dy, dz);
+        u64 ck;
+        if constexpr (BATCH) ck = pack_cell_batch(scene, ux + dx, uy + dy, uz + dz);
+        else ck = pack_cell(ux + dx, uy + dy, uz + dz);
+        const u32 slot = find_slot<BATCH>(a.fluid.table, a.fluid.tmask, ck);
+        if (slot == EMPTY_CELL) continue;
+        const u32 e = ro_ld(a.fluid.cend + slot);
+        for (u32 j = ro_ld(a.fluid.cstart + slot); j < e; ++j) {
+            const float r2 = dist2(xi, ro_ld(a.pos + guard(a, j, a.n)));
+            if (!(r2 <= P.h2) || j == i) continue;
+            if (hits < a.nbr_width) a.nbr[hits * a.n + i] = j;
+            ++hits;
+            density_pair(r2, P, t3, u3);
+        }
+    }
+    return hits;
+}
+
+// Neighbours of row i among the staged candidates. seg0: first cell of the
+// row's 9 runs (the block's cell grid has Dy x Dz cells per x); selfm: the
+// row's own candidate index. Returns the neighbour count.
+template <class C>
+__device__ __forceinline__ u32 density_staged_row(const DevParams& P, const TravArgs& a, BlockSmem<C>& S, u32 i,
+                                                  float4 xi, u32 seg0, u32 Dy, u32 Dz, u32 selfm, bool act, float& t3,
+                                                  float& u3) {
+    const float2 nx = make_float2(-xi.x, -xi.x), ny = make_float2(-xi.y, -xi.y), nz = make_float2(-xi.z, -xi.z);
+    const float lim = -__uint_as_float(__float_as_uint(P.h2) + 1u);   // minus the float after h2
+    const float2 nlim = make_float2(lim, lim);
+    u32* const word = S.word + threadIdx.x;
+    unsigned short* const wbase = S.wbase + threadIdx.x;
+    u32 hits = 0;
+    u32 slot_idx = i;      // list slot of the next hit (u32: the host caps nbr_width * n below 2^32)
+    u32 seg = act ? 0u : 9u;
+    u32 b = 0, s0 = 0, e0 = 0;
+    bool open = false;     // segment seg is partly tested: [b, e0) remains
+    do {
+        // phase 1: words with hits, until all segments are tested or the column is full
+        u32 k = 0;
+        while (seg < 9u && k < static_cast<u32>(C::words)) {
+            if (!open) {
+                const u32 c = seg0 + ((seg / 3u) * Dy + seg % 3u) * Dz;
+                s0 = S.rpref[c];
+                e0 = S.rpref[c + 3u];
+                b = s0 & ~3u;
+            }
+            if (b < e0) {
+                                const u32 nq = min(8u, (e0 - b + 3u) >> 2);
+                const float4* X = reinterpret_cast<const float4*>(S.x + b);
+                const float4* Y = reinterpret_cast<const float4*>(S.y + b);
+                const float4* Z = reinterpret_cast<const float4*>(S.z + b);
+                u32 bits = 0;
+#pragma unroll
+                for (u32 q = 0; q < 8u; ++q) {
+                    if (q >= nq) break;
+                    const float4 cx = X[q], cy = Y[q], cz = Z[q];
+                    // x_j - x_i: the square is that of x_i - x_j, bit for bit
+                    const float2 dx0 = __fadd2_rn(make_float2(cx.x, cx.y), nx);
+                    const float2 dx1 = __fadd2_rn(make_float2(cx.z, cx.w), nx);
+                    const float2 dy0 = __fadd2_rn(make_float2(cy.x, cy.y), ny);
+                    const float2 dy1 = __fadd2_rn(make_float2(cy.z, cy.w), ny);
+                    const float2 dz0 = __fadd2_rn(make_float2(cz.x, cz.y), nz);
+                    const float2 dz1 = __fadd2_rn(make_float2(cz.z, cz.w), nz);
+                    const float2 r0 = __fadd2_rn(__ffma2_rn(dz0, dz0, __ffma2_rn(dx0, dx0, __fmul2_rn(dy0, dy0))), nlim);
+                    const float2 r1 = __fadd2_rn(__ffma2_rn(dz1, dz1, __ffma2_rn(dx1, dx1, __fmul2_rn(dy1, dy1))), nlim);
+                    bits = __funnelshift_l(__float_as_uint(r0.x), bits, 1);
+                    bits = __funnelshift_l(__float_as_uint(r0.y), bits, 1);
+                    bits = __funnelshift_l(__float_as_uint(r1.x), bits, 1);
+                    bits = __funnelshift_l(__float_as_uint(r1.y), bits, 1);
+                }
+                bits <<= 32u - 4u * nq;          // candidate b + t at bit 31 - t
+                if (b < s0) bits &= FULL >> (s0 - b);
+                if (e0 - b < 32u) bits &= ~(FULL >> (e0 - b));
+                const u32 me = selfm - b;
+                if (me < 32u) bits &= ~(0x80000000u >> me);
+                if (bits) {
+                    hits += __popc(bits);
+                    word[k * C::nt] = bits;
+                    wbase[k * C::nt] = static_cast<unsigned short>(b);
+                    ++k;
+                }
+                b += 32u;
+            }
+            open = b < e0;
+            if (!open) ++seg;
+        }
+        // phase 2: the hits, in candidate order
+        const bool listed = hits <= a.nbr_width;   // else the row's list is not used
+        if (k) {
+            u32 t = 0;
+            u32 w = word[0];
+            u32 base = wbase[0];
+            do {
+                const u32 bit = static_cast<u32>(__clz(static_cast<int>(w)));
+                const u32 m = guard(a, base + bit, C::cap);
+                w ^= 0x80000000u >> bit;
+                if (w == 0u && ++t < k) {
+                    w = word[t * C::nt];
+                    base = wbase[t * C::nt];
+                }
+                const float r2 = dist2(xi, make_float4(S.x[m], S.y[m], S.z[m], 0.f));
+                if (listed) a.nbr[slot_idx] = S.j[m];
+                slot_idx += a.n;
+                density_pair(r2, P, t3, u3);
+            } while (w);
+        }
+    } while (seg < 9u);
+    return hits;
+}
+
+// The particles of the block that starts at sorted index `start`, by the whole
+// thread block.
+template <class C, bool BATCH>
+__device__ __forceinline__ void density_unit(const DevParams& P, const TravArgs& a, BlockSmem<C>& S, u32 start) {
+    const u32 tid = threadIdx.x;
+    const u32 lane = tid & 31u;
+    const u32 n = a.n;
+    u32 level = a.unit_level;
+    const u64 unit_mask = block_mask<BATCH>(level);
+    u32 i0 = start;
+    const u64 unit_id = a.ckey[i0] & unit_mask;
+    for (;;) {
+        const u64 pk0 = a.ckey[i0];
+        const u64 mask = block_mask<BATCH>(level);
+        const u64 id = pk0 & mask;
+        u32 ux, uy, uz, scene;
+        decode_cell<BATCH>(id, ux, uy, uz, scene);
+        const u32 lx = (level + 2u) / 3u, ly = (level + 1u) / 3u, lz = level / 3u;
+        const u32 ox = ux - 1u, oy = uy - 1u, oz = uz - 1u;   // first cell of the surrounding layer
+        const u32 Dx = (1u << lx) + 2u, Dy = (1u << ly) + 2u, Dz = (1u << lz) + 2u;
+        const u32 ncell = Dx * Dy * Dz;
+        // keys of the first rows, in flight during the lookups
+        u64 rk[3];
+#pragma unroll
+        for (u32 k = 0; k < 3u; ++k) {
+            const u32 i = i0 + k * C::nt + tid;
+            rk[k] = i < n ? a.ckey[i] : ~id;
+        }
+        // cells of the block and its layer: start and count
+        for (u32 q = tid; q < ncell; q += C::nt) {
+            const u32 x = q / (Dy * Dz), y = (q / Dz) % Dy, z = q % Dz;
+            u64 pk;
+            if constexpr (BATCH) pk = pack_cell_batch(scene, ox + x, oy + y, oz + z);
+            else pk = pack_cell(ox + x, oy + y, oz + z);
+            const u32 slot = find_slot<BATCH>(a.fluid.table, a.fluid.tmask, pk);
+            u32 s = 0, cnt = 0;
+            if (slot != EMPTY_CELL) {
+                s = ro_ld(a.fluid.cstart + slot);
+                const u32 e = ro_ld(a.fluid.cend + slot);
+                cnt = e > s ? e - s : 0u;
+            }
+            S.rstart[q] = s;
+            S.rpref[q] = cnt;
+        }
+        // rows of the block: the run of equal block keys from i0 on
+        u32 rows = 0;
+        for (u32 base = i0;;) {
+            bool more = true;
+#pragma unroll
+            for (u32 k = 0; k < 3u; ++k) {
+                if (!more) continue;
+                const u32 c = static_cast<u32>(__syncthreads_count((rk[k] & mask) == id));
+                rows += c;
+                more = c == static_cast<u32>(C::nt);
+            }
+            if (!more) break;
+            base += 3u * C::nt;
+#pragma unroll
+            for (u32 k = 0; k < 3u; ++k) {
+                const u32 i = base + k * C::nt + tid;
+                rk[k] = i < n ? a.ckey[i] : ~id;
+            }
+        }
+        // exclusive prefix of the counts (the barrier above made them visible)
+        if (tid < 32u) {
+            u32 run = 0;
+            for (u32 base = 0; base < ncell; base += 32u) {
+                const u32 q = base + lane;
+                const u32 c = q < ncell ? S.rpref[q] : 0u;
+                const u32 incl = warp_incl_scan(c);
+                if (q < ncell) S.rpref[q] = run + incl - c;
+                run += __shfl_sync(FULL, incl, 31);
+            }
+            if (lane == 0) S.rpref[ncell] = run;
+        }
+        __syncthreads();
+        const u32 M = S.rpref[ncell];
+        if (M > static_cast<u32>(C::cap) && level > 0u) {   // too dense: smaller blocks, same thread block
+            --level;
+            __syncthreads();
+            continue;
+        }
+        const bool staged = M <= static_cast<u32>(C::cap);
+        if (staged) {
+            // eight lanes per cell: a cell's particles are contiguous
+            for (u32 q = tid >> 3; q < ncell; q += C::nt / 8) {
+                const u32 s = S.rstart[q], m0 = S.rpref[q], cnt = S.rpref[q + 1u] - m0;
+                for (u32 t = tid & 7u; t < cnt; t += 8u) {
+                    const u32 j = guard(a, s + t, n);
+                    const float4 p = ro_ld(a.pos + j);
+                    const u32 m = guard(a, m0 + t, C::cap);
+                    S.x[m] = p.x;
+                    S.y[m] = p.y;
+                    S.z[m] = p.z;
+                    S.j[m] = j;
+                }
+            }
+        }
+        __syncthreads();
+        for (u32 r0 = tid & ~31u; r0 < rows; r0 += C::nt) {
+            const u32 r = r0 + lane;
+            const bool act = r < rows;
+            const u32 i = i0 + (act ? r : 0u);
+            const u64 pk = a.ckey[i];
+            const float4 xi = ro_ld(a.pos + guard(a, i, n));
+            float t3 = 0.f, u3 = 0.f;
+            u32 hits = 0;
+            if (staged) {
+                u32 cx, cy, cz, sc;
+                decode_cell<BATCH>(pk, cx, cy, cz, sc);
+                cx -= ox; cy -= oy; cz -= oz;   // 1 .. D - 2 per axis
+                const u32 cell = guard(a, (cx * Dy + cy) * Dz + cz, ncell);
+                const u32 s = S.rstart[cell], m0 = S.rpref[cell];
+                const u32 selfm = i - s < S.rpref[cell + 1u] - m0 ? m0 + (i - s) : 0xFFFF0000u;
+                hits = density_staged_row<C>(P, a, S, i, xi, cell - (Dy + 1u) * Dz - 1u, Dy, Dz, selfm, act, t3, u3);
+            } else if (act) {
+                hits = density_direct_row<BATCH>(P, a, i, pk, xi, t3, u3);
+            }
+            if (act) {
+                const float res[1] = {__fmaf_rn(2.f, t3, -u3)};
+                float resb[1] = {0.f};
+                if (a.nb > 0) density_boundary_row<BATCH>(P, a, xi, scene, i, resb);
+                float r_max = 0.f, r_s = 0.f, r_s2 = 0.f;
+                finish_row<PASS_DENSITY, BATCH>(P, a, i, res, resb, hits <= a.nbr_width ? hits : NBR_SPILL, scene, 0.f,
+                                                0.f, r_max, r_s, r_s2);
+            }
+        }
+        if (level == a.unit_level) return;
+        i0 += rows;
+        if (i0 >= n || (a.ckey[i0] & unit_mask) != unit_id) return;   // the same for every thread
+        __syncthreads();
+    }
+}
+
+// Units of the whole array, claimed from a device counter (the next claim is
+// in flight while a unit is worked on). The list and both counters are
+// rebuilt by the sort plan and the reorder of every step.
+template <class C, bool BATCH>
+__device__ __forceinline__ void density_units(const DevParams& P, const TravArgs& a, BlockSmem<C>& S) {
+    const u32 count = *reinterpret_cast<const volatile u32*>(&a.st->unit_count);
+    u32 u = blockIdx.x;   // the first claim of every block is its own index
+    while (u < count) {
+        u32 nxt = 0;
+        if (threadIdx.x == 0) nxt = atomicAdd(&a.st->unit_next, 1u) + gridDim.x;
+        density_unit<C, BATCH>(P, a, S, guard(a, a.units[u], a.n));
+        __syncthreads();
+        if (threadIdx.x == 0) S.next = nxt;
+        __syncthreads();
+        u = S.next;
+    }
+}
+
+}  // namespace
+}  // namespace wcsph

@@ -304,8 +304,10 @@ TravArgs CUDASPHSimulator::trav_args(float delta) {
     a.mask = mask_.ptr;
     a.mask_words = static_cast<u32>(cfg_.mask_words);
     a.chunk = effective_chunk(cfg_, n_);
+    a.units = use_units() ? unit_buf() : nullptr;
+    a.unit_level = unit_level(n_);
     a.nbr = nbr_width_ > 0 ? nbr_.ptr : nullptr;
-    a.pair_cells = a.nbr != nullptr ? 1u : 0u;   // the lists replace the kept bit matrix
+    a.keep_matrix = a.nbr == nullptr ? 1u : 0u;   // the lists replace the kept bit matrix
     a.matrix_valid = 0u;
     a.nbr_cnt = nbr_cnt_.ptr;
     a.nbr_width = nbr_width_;
@@ -339,7 +341,7 @@ void CUDASPHSimulator::enqueue_search(bool keys_from_state) {
     WCSPH_CUDA(enqueue_sort_passes(sb, n, st_.ptr, stream_));
     launch_reorder_cells(pos_a_.ptr, vel_a_.ptr, vals_[1].ptr, vals_[2].ptr, st_.ptr, n, dp_.cell_size, pos_b_.ptr,
                          vel_b_.ptr, perm_.ptr, ckey_.ptr, table_.ptr, cstart_.ptr, cend_.ptr, table_size_ - 1,
-                         st_.ptr, stream_);
+                         st_.ptr, stream_, nullptr, use_units() ? unit_buf() : nullptr, unit_level(n_));
 }
 
 void CUDASPHSimulator::enqueue_keys() {
@@ -358,7 +360,8 @@ TravArgs CUDASPHSimulator::fixed_args(float dt) {
     a.cfl_factor = 0.f;
     a.max_dt = dt;
     a.min_dt = dt;
-    a.pair_cells = 0u;   // the adjoint passes walk each step's kept bit matrix
+    a.keep_matrix = 1u;   // the adjoint passes walk each step's kept bit matrix
+    a.units = nullptr;
     return a;
 }
 
@@ -675,7 +678,7 @@ int CUDASPHSimulator::kernel_timings(const char** names, float* ms, int cap) {
     WCSPH_CUDA(cudaEventRecord(ev[2], stream_));
     launch_reorder_cells(pos_a_.ptr, vel_a_.ptr, vals_[1].ptr, vals_[2].ptr, st_.ptr, n, dp_.cell_size, pos_b_.ptr,
                          vel_b_.ptr, perm_.ptr, ckey_.ptr, table_.ptr, cstart_.ptr, cend_.ptr, table_size_ - 1,
-                         st_.ptr, stream_);
+                         st_.ptr, stream_, nullptr, use_units() ? unit_buf() : nullptr, unit_level(n_));
     WCSPH_CUDA(cudaEventRecord(ev[3], stream_));
     const TravArgs a = trav_args(delta);
     launch_pass(PASS_DENSITY, dp_, a, stream_, cfg_.warps_density);

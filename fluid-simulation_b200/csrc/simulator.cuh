@@ -193,6 +193,11 @@ private:
     TravArgs trav_args(float delta);
     u32 fluid_table_size() const;
     void ensure_tables();
+    // The density pass works on blocks of cells (density_blocks.cuh) where the
+    // lists are on and the neighbourhood is one cell deep.
+    bool use_units() const { return nbr_width_ > 0 && dp_.range == 1; }
+    // Unit list: the sort's second key buffer, free once the sort is done.
+    u32* unit_buf() { return reinterpret_cast<u32*>(keys_[1].ptr); }
 
     friend class Tuner;
     friend struct Adjoint;

@@ -229,6 +229,16 @@ __host__ __device__ __forceinline__ u64 cell_hash_batch(u64 pk) {
     return cell_hash(static_cast<u32>(pk & 0xFFFFull), static_cast<u32>((pk >> 16) & 0xFFFFull),
                      static_cast<u32>((pk >> 32) & 0xFFFFull)) ^ (0x9E3779B97F4A7C15ull * s);
 }
+// Packed cell key bits that name the Morton-aligned block of 2^level cells
+// (x, y, z halved in turn from the whole block down) a cell lies in: clears the
+// low ceil(level / 3), ceil((level - 1) / 3), level / 3 bits of x, y, z.
+template <bool BATCH>
+__host__ __device__ __forceinline__ u64 block_mask(u32 level) {
+    constexpr u32 w = BATCH ? 16u : 21u;
+    const u64 x = (1ull << ((level + 2u) / 3u)) - 1u, y = (1ull << ((level + 1u) / 3u)) - 1u,
+              z = (1ull << (level / 3u)) - 1u;
+    return ~(x | (y << w) | (z << (2u * w)));
+}
 template <bool BATCH>
 __host__ __device__ __forceinline__ u64 slot_hash(u64 pk) {
     if constexpr (BATCH) return cell_hash_batch(pk);
@@ -299,7 +309,10 @@ struct DevState {
     u32 sort_sel[9];            // buffer read by pass p; sort_sel[8] = final
     u32 sort_tile_counter[8];
     u32 first_active;           // first active pass (generates the iota values)
-    u32 pad1[2];
+    // density units (blocks of cells): listed by the reorder, claimed by the
+    // density pass; both reset by the sort plan
+    u32 unit_count;
+    u32 unit_next;
     // cell-coordinate bounds of the particles of the current sort (0 is always
     // included; reset to 0 by the sort plan): they choose the compressed keys
     int cell_lo[3];

@@ -61,10 +61,10 @@ __device__ __forceinline__ T ro_ld(const T* p) {
 }
 
 __device__ __forceinline__ u32 guard(const TravArgs& a, u32 idx, u32 bound) { return guard_st(a.st, idx, bound); }
-// Cells of the staged neighbourhood ranges: (2R + 1)^3, or the 36 of an x-pair union.
+// Cells of the staged neighbourhood ranges: (2R + 1)^3.
 __device__ __forceinline__ u32 range_cells(const TravArgs& a) {
     const u32 d = 2u * static_cast<u32>(a.range) + 1u;
-    return max(d * d * d, 36u);
+    return d * d * d;
 }
 
 // Linear-probed lookup of a packed cell key (find_cell_in_table,
@@ -86,15 +86,7 @@ constexpr u32 FULL = 0xffffffffu;
 constexpr u32 BCAND_CAP = 256;   // boundary candidates expanded per warp and chunk
 constexpr u32 HOME_BLOCK = 32;   // home particles (bit-matrix rows) handled together
 constexpr u32 SEG_SLOTS = 64;    // segment partials, slot = lane + row (both < 32)
-constexpr u32 NO_HOME = 0xFFFFFFFFu;   // home rows not among the staged candidates
-
-// Candidate index of home row k of a home block: rows [0, split) are staged
-// at c1 + k, later rows at c2 + (k - split) (the second cell of an x-pair);
-// c1 == NO_HOME: the home rows are not staged (read from global memory).
-struct HomeMap {
-    u32 split, c1, c2;
-    __device__ __forceinline__ u32 cand(u32 k) const { return k < split ? c1 + k : c2 + (k - split); }
-};
+constexpr u32 NO_HOME = 0xFFFFFFFFu;   // home rows not among the staged candidates (read from global memory)
 
 
 __device__ __forceinline__ u32 lane_id() { return threadIdx.x & 31u; }
@@ -177,10 +169,8 @@ __host__ __device__ __forceinline__ size_t warp_smem_bytes(u32 cap, u32 ncell, b
     unsigned char* sp = C::soa ? take(8ull * pair_slot(cap / 2)) : nullptr;
     unsigned char* cand = C::stage_j ? take(4ull * cap) : nullptr;
     unsigned char* cq = C::stage_q ? take(cap) : nullptr;
-    // density: room for the 36-cell union of an x-pair of cells (R = 1)
-    const u32 nrange = (KIND == PASS_DENSITY && ncell < 36u) ? 36u : ncell;
-    unsigned char* rstart = take(4ull * (nrange + 3));
-    unsigned char* rpref = take(4ull * (nrange + 3));
+    unsigned char* rstart = take(4ull * (ncell + 3));
+    unsigned char* rpref = take(4ull * (ncell + 3));
     unsigned char *bcand = nullptr, *bstart = nullptr, *bpref = nullptr;
     if (C::boundary && with_boundary) {   // only scenes with boundary particles
         bcand = take(4ull * BCAND_CAP);
@@ -293,8 +283,7 @@ __device__ __forceinline__ void stage(const WarpView<KIND>& S, const TravArgs& a
     const u32 lane = lane_id();
     const u32 c1 = c0 + len;
     for (u32 qb = 0; qb < ncell; qb += 32) {
-        // a last round of fewer than 32 cells (the 36-cell union of an x-pair)
-        // spreads each cell over 32 / cells lanes
+        // a last round of fewer than 32 cells spreads each cell over 32 / cells lanes
         const u32 rem = min(32u, ncell - qb);
         const u32 lpc = rem == 32u ? 1u : 32u / rem;
         const u32 q = qb + lane / lpc;
@@ -703,12 +692,11 @@ __device__ __forceinline__ u32 fluid_pair_run(const WarpView<KIND>& S, const Dev
 }
 
 // Position of home row k of the density pass: from the staged candidates
-// (hm maps rows to candidate indices) when they hold the home cells, else
-// from global memory.
-__device__ __forceinline__ float4 home_x(const WarpView<PASS_DENSITY>& S, const TravArgs& a, u32 i0, HomeMap hm,
-                                         u32 k) {
-    if (hm.c1 != NO_HOME) {
-        const u32 m = guard(a, hm.cand(k), a.mask_words * 32u);
+// (row 0 is candidate c0) when they hold the home cell, else (NO_HOME) from
+// global memory.
+__device__ __forceinline__ float4 home_x(const WarpView<PASS_DENSITY>& S, const TravArgs& a, u32 i0, u32 c0, u32 k) {
+    if (c0 != NO_HOME) {
+        const u32 m = guard(a, c0 + k, a.mask_words * 32u);
         const float* f = reinterpret_cast<const float*>(S.sp + pair_slot(m >> 1)) + (m & 1u);
         return make_float4(f[0], f[2], f[4], 0.f);
     }
@@ -723,12 +711,12 @@ __device__ __forceinline__ float4 home_x(const WarpView<PASS_DENSITY>& S, const 
 template <int KIND, bool SHARED_BITS = false>
 __device__ __forceinline__ u32 fluid_hit_run(const WarpView<KIND>& S, const DevParams& P, const TravArgs& a,
                                              const u32* WCSPH_RESTRICT bits, u32 nh, u32 M, u32 i0, u32& lo,
-                                             u32& hi, bool lists = false, HomeMap hm = HomeMap{32u, NO_HOME, 0u}) {
+                                             u32& hi, bool lists = false, u32 c0 = NO_HOME) {
     auto home = [&](u32 k) -> HomeData {
         if constexpr (KIND == PASS_DENSITY) {
-            if (hm.c1 != NO_HOME) {
+            if (c0 != NO_HOME) {
                 HomeData H;
-                H.x = home_x(S, a, i0, hm, k);
+                H.x = home_x(S, a, i0, c0, k);
                 return H;
             }
         }
@@ -825,12 +813,8 @@ __device__ __forceinline__ u32 fluid_hit_run(const WarpView<KIND>& S, const DevP
 // unrolled, each tested in packed FP32 with the rounding of dist2()
 // (x_i - x_j is formed as fma(x_j, -1, x_i), the same single rounding).
 // The home particle's own bit is set here and cleared by the caller.
-// Row windows: rows [0, hm.split) keep candidates [0, win_a) only, later rows
-// [win_b, 32 wpr) only (the two cells of an x-pair, each restricted to its own
-// 27 neighbour cells; a single cell passes win_a = 32 wpr).
 __device__ __forceinline__ void density_test_words(const WarpView<PASS_DENSITY>& S, const DevParams& P,
-                                                   const TravArgs& a, u32 nh, u32 wpr, u32 i0, HomeMap hm,
-                                                   u32 win_a, u32 win_b) {
+                                                   const TravArgs& a, u32 nh, u32 wpr, u32 i0, u32 c0) {
     const u32 nwords = nh * wpr;
     const float2 neg = make_float2(-1.f, -1.f);
     // w / wpr as a multiply-high: exact for w < 2^32 / wpr^2 (here w < 32 * 16)
@@ -838,7 +822,7 @@ __device__ __forceinline__ void density_test_words(const WarpView<PASS_DENSITY>&
     for (u32 w = lane_id(); w < nwords; w += 32) {
         const u32 k = wpr == 1u ? w : __umulhi(w, inv);
         const u32 wi = w - k * wpr;
-        const float4 h = home_x(S, a, i0, hm, k);
+        const float4 h = home_x(S, a, i0, c0, k);
         const float2 X = make_float2(h.x, h.x), Y = make_float2(h.y, h.y), Z = make_float2(h.z, h.z);
         const float2* base = S.sp + pair_slot(wi * 16u);
         u32 bits = 0;
@@ -850,11 +834,6 @@ __device__ __forceinline__ void density_test_words(const WarpView<PASS_DENSITY>&
             const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
             bits |= (r2.x <= P.h2 ? 1u << (2 * t) : 0u) | (r2.y <= P.h2 ? 2u << (2 * t) : 0u);
         }
-        // candidates [lo, hi) of the row's window within this word
-        const u32 lo = k < hm.split ? 0u : win_b, hi = k < hm.split ? win_a : 0xFFFFFFFFu;
-        const u32 w0 = wi << 5;
-        if (lo > w0) bits &= lo >= w0 + 32u ? 0u : FULL << (lo - w0);
-        if (hi < w0 + 32u) bits &= hi <= w0 ? 0u : FULL >> (w0 + 32u - hi);
         S.aux[w] = bits;
     }
     __syncwarp();
@@ -898,39 +877,23 @@ __device__ __forceinline__ u32 boundary_pair_run(const WarpView<KIND>& S, const 
     return c;
 }
 
-// Boundary pairs of rows [0, nh) from per-cell candidate runs: rows
-// [0, split) against run A = [sa, sa + la) of bcx, later rows against run
-// B = [sb, sb + lb) (the second cell of an x-pair). Segmented like
-// boundary_pair_run; returns the run length and, for row k = lane, its item
-// range [lo, hi).
+// Boundary pairs of rows [0, nh) of one cell from its candidate run [run,
+// run + len) of bcx. Segmented like boundary_pair_run; returns the run length.
 // masks (density, a.bmask): hit m < 128 of row k also sets bit m of
 // S.aux[4k .. 4k + 3], which the caller zeroes before and stores after.
 template <int KIND>
 __device__ __forceinline__ u32 boundary_cells_run(const WarpView<KIND>& S, const DevParams& P, const TravArgs& a,
-                                                  u32 nh, u32 i0, u32 split, u32 sa, u32 la, u32 sb, u32 lb,
-                                                  u32& lo, u32& hi, bool masks = false) {
+                                                  u32 nh, u32 i0, u32 run, u32 len, bool masks = false) {
     constexpr int NFB = KindCfg<KIND>::nfb;
     const u32 lane = lane_id();
-    const u32 na = split * la;
-    const u32 total = na + (nh - split) * lb;
-    lo = lane < split ? lane * la : na + (min(lane, nh) - split) * lb;
-    hi = lo + (lane < nh ? (lane < split ? la : lb) : 0u);
+    const u32 total = nh * len;
     if (total == 0) return 0;
     const u32 c = ((total + 31u) >> 5) | 1u;
     u32 p = lane * c;
     const u32 e = min(p + c, total);
     if (p < e) {
-        u32 k, m;
-        if (p < na) {
-            k = p / la;
-            m = p - k * la;
-        } else {
-            const u32 q = p - na;
-            k = split + q / lb;
-            m = q - (k - split) * lb;
-        }
-        u32 len = k < split ? la : lb;
-        u32 run = k < split ? sa : sb;
+        u32 k = p / len;
+        u32 m = p - k * len;
         HomeData H = load_home<KIND>(a, i0 + k);
         float v[NFB];
 #pragma unroll
@@ -950,8 +913,6 @@ __device__ __forceinline__ u32 boundary_cells_run(const WarpView<KIND>& S, const
                 for (int f = 0; f < NFB; ++f) v[f] = 0.f;
                 m = 0;
                 ++k;
-                len = k < split ? la : lb;
-                run = k < split ? sa : sb;
                 H = load_home<KIND>(a, i0 + k);
             }
         }
@@ -1365,72 +1326,16 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                 uy = static_cast<u32>((pk >> 21) & 0x1FFFFFull);
                 uz = static_cast<u32>((pk >> 42) & 0x1FFFFFull);
             }
-            // Density with lists: a cell of even x and the cell of x + 1 after
-            // it (Morton-consecutive, so adjacent in sorted order whenever both
-            // are occupied) form an x-pair, handled whole by the warp of the
-            // first: one lookup of the union of their neighbour cells (4 x 3 x 3,
-            // in the reference's x, y, z order), one staging, and twice the
-            // home rows per walk. The warp of the second cell skips it.
-            bool pair_try = false;
-            if constexpr (KIND == PASS_DENSITY) {
-                if (a.pair_cells && R == 1) {
-                    if (ux & 1u) {
-                        u64 apk;
-                        if constexpr (BATCH) apk = pack_cell_batch(scene, ux - 1u, uy, uz);
-                        else apk = pack_cell(ux - 1u, uy, uz);
-                        if (__shfl_sync(FULL, prev_pk, s) == apk && base + s > 0) continue;
-                    } else {
-                        pair_try = true;
-                    }
-                }
-            }
-            u32 gx = ux;   // x of the cell whose neighbourhood is gathered
-            auto gather = [&](u32 nc) {
-                return gather_ranges<BATCH>(S.rstart, S.rpref, nc, a.fluid, [&](u32 q) {
-                    int dx, dy, dz;
-                    cell_offset(q, R, dx, dy, dz);   // R = 1: q < 36 gives dx in [-1, 2]
-                    if constexpr (BATCH) return pack_cell_batch(scene, gx + dx, uy + dy, uz + dz);
-                    else return pack_cell(gx + dx, uy + dy, uz + dz);
-                });
-            };
-            u32 units = 1;
-            for (u32 unit = 0; unit < units; ++unit) {
             // fluid neighbour cells in the reference's x, y, z nesting order
-            u32 M, ncs, home_start, n_home, self_base;
-            bool pair = false;
-            u32 nA = 0, selfB = 0, winA = 0, winB = 0;
-            if (unit == 0) {
-                M = gather(pair_try ? 36u : ncell);
-                ncs = ncell;
-                home_start = S.rstart[qc];
-                n_home = S.rpref[qc + 1] - S.rpref[qc];
-                self_base = S.rpref[qc];   // candidate index of the first home particle
-                if (pair_try) {
-                    // union cells 0..26: the first cell's neighbourhood, 9..35: the second's
-                    nA = n_home;
-                    const u32 nB = S.rpref[23] - S.rpref[22];
-                    const bool second = nB > 0 && S.rstart[22] == home_start + nA;
-                    if (second && ((M + 31u) & ~31u) <= a.mask_words * 32u) {
-                        pair = true;
-                        ncs = 36;
-                        n_home = nA + nB;
-                        selfB = S.rpref[22];
-                        winA = S.rpref[27];
-                        winB = S.rpref[9];
-                    } else {
-                        M = S.rpref[27];   // the first cell alone (its 27 cells lead the union)
-                        if (second) units = 2;
-                    }
-                }
-            } else {
-                // the second cell of a pair whose union exceeds the bit-matrix capacity
-                gx = ux + 1u;
-                M = gather(ncell);
-                ncs = ncell;
-                home_start = S.rstart[qc];
-                n_home = S.rpref[qc + 1] - S.rpref[qc];
-                self_base = S.rpref[qc];
-            }
+            const u32 M = gather_ranges<BATCH>(S.rstart, S.rpref, ncell, a.fluid, [&](u32 q) {
+                int dx, dy, dz;
+                cell_offset(q, R, dx, dy, dz);
+                if constexpr (BATCH) return pack_cell_batch(scene, ux + dx, uy + dy, uz + dz);
+                else return pack_cell(ux + dx, uy + dy, uz + dz);
+            });
+            const u32 home_start = S.rstart[qc];
+            const u32 n_home = S.rpref[qc + 1] - S.rpref[qc];
+            const u32 self_base = S.rpref[qc];   // candidate index of the first home particle
             const u32 Mrow = (M + 31u) & ~31u;     // bit-matrix row length (whole words)
             const bool masked = Mrow <= cap;
 
@@ -1439,19 +1344,15 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
             // for_boundary_neighbors common.cuh:153-178)
             u32 MB = 0, nbc = 0;
             // density with per-cell boundary candidates (cell size h): the
-            // runs of the unit's home cells (A, and B of an x-pair)
+            // home cell's run
             const bool use_cells = KIND == PASS_DENSITY && a.bcell.table != nullptr && P.cell_size == P.h;
-            u32 bra = 0, bla = 0, brb = 0, blb = 0;
+            u32 brun = 0, blen = 0;
             if (use_cells && a.nb > 0) {
                 u32 s0 = 0, s1 = 0;
-                if (lane < (pair ? 2u : 1u)) {
-                    const int3 hc = cell_of(a.pos[home_start + (lane ? nA : 0u)], P.h);
-                    boundary_run<BATCH>(a, boundary_cell_key<BATCH>(hc, scene), s0, s1);
-                }
-                bra = __shfl_sync(FULL, s0, 0);
-                bla = __shfl_sync(FULL, s1, 0) - bra;
-                brb = __shfl_sync(FULL, s0, 1);
-                blb = __shfl_sync(FULL, s1, 1) - brb;
+                if (lane == 0)
+                    boundary_run<BATCH>(a, boundary_cell_key<BATCH>(cell_of(a.pos[home_start], P.h), scene), s0, s1);
+                brun = __shfl_sync(FULL, s0, 0);
+                blen = __shfl_sync(FULL, s1, 0) - brun;
             }
             if constexpr (C::boundary) {
                 if (a.nb > 0 && !use_cells) {
@@ -1485,7 +1386,7 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                 }
             }
 
-            if (masked) stage<KIND>(S, a, ncs, 0, M);
+            if (masked) stage<KIND>(S, a, ncell, 0, M);
             // the cell's neighbour bit matrix: row k = home particle k, bit m = candidate m
             u32* const cell_bits = a.mask + static_cast<size_t>(home_start) * a.mask_words;
 
@@ -1493,10 +1394,6 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                 const u32 nh = min(HOME_BLOCK, n_home - hb);
                 const u32 i0 = home_start + hb;
                 const u32 self0 = self_base + hb;
-                // candidate index of each home row of the block (x-pairs: the
-                // rows of the second cell follow those of the first)
-                const HomeMap hm = pair ? HomeMap{nA > hb ? nA - hb : 0u, self0, selfB + (hb > nA ? hb - nA : 0u)}
-                                        : HomeMap{32u, self0, 0u};
                 const bool act = lane < nh;
                 const u32 i = i0 + (act ? lane : 0u);
                 u32* const blk_bits = cell_bits + (hb >> 5) * Mrow;   // row hb starts at bit hb * Mrow
@@ -1535,7 +1432,7 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                         const float4 xi = a.pos[i];
                         for (u32 c0 = 0; c0 < M; c0 += cap) {
                             const u32 len = min(cap, M - c0);
-                            stage<KIND>(S, a, ncs, c0, len);
+                            stage<KIND>(S, a, ncell, c0, len);
                             if (act) {
                                 for (u32 ml = 0; ml < len; ++ml) {
                                     if (c0 + ml != self0 + lane && dist2(xi, S.sa[ml]) <= P.h2) {
@@ -1561,10 +1458,9 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                         const u32 wpr = (len + 31u) >> 5;
                         const u32 len32 = wpr << 5;
                         const u32 nwords = nh * wpr;
-                        // masked: the home cells are staged
-                        const HomeMap hmc = keep_bits ? hm : HomeMap{32u, NO_HOME, 0u};
-                        density_test_words(S, P, a, nh, wpr, i0, hmc, pair ? winA : len32, winB);
-                        const u32 self = (keep_bits ? hm.cand(lane) : self0 + lane) - c0;   // the home particle itself
+                        const u32 hc0 = keep_bits ? self0 : NO_HOME;   // masked: the home cell is staged
+                        density_test_words(S, P, a, nh, wpr, i0, hc0);
+                        const u32 self = self0 + lane - c0;   // the home particle itself
                         if (act && self < len) {
                             const u32 item = lane * len32 + self;
                             atomicAnd(S.aux + (item >> 5), ~(1u << (item & 31u)));
@@ -1572,10 +1468,10 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                         __syncwarp();
                         u32 lo, hi;
                         const u32 c = fluid_hit_run<KIND, true>(S, P, a, S.aux, nh, len32, i0, lo, hi,
-                                                                keep_bits && a.nbr != nullptr, hmc);
+                                                                keep_bits && a.nbr != nullptr, hc0);
                         if (c) combine<NF>(S.part, res, act, lo, hi, c, lane);
                         if (keep_bits && hi - lo <= a.nbr_width) row_cnt = hi - lo;
-                        if (keep_bits && !a.pair_cells)   // kept for the neighbour export and the adjoint
+                        if (keep_bits && a.keep_matrix)   // read by the later passes
                             for (u32 w = lane; w < nwords; w += 32) blk_bits[w] = S.aux[w];
                         __syncwarp();
                     };
@@ -1584,7 +1480,7 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                     } else {
                         for (u32 c0 = 0; c0 < M; c0 += cap) {
                             const u32 len = min(cap, M - c0);
-                            stage<KIND>(S, a, ncs, c0, len);
+                            stage<KIND>(S, a, ncell, c0, len);
                             density_chunk(c0, len, false);
                         }
                     }
@@ -1600,7 +1496,7 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                     } else {
                         for (u32 c0 = 0; c0 < M; c0 += cap) {
                             const u32 len = min(cap, M - c0);
-                            stage<KIND>(S, a, ncs, c0, len);
+                            stage<KIND>(S, a, ncell, c0, len);
                             const u32 c = fluid_pair_run<KIND>(S, P, a, nh, len, c0, i0, self0);
                             combine<NF>(S.part, res, act, lane * len, lane * len + len, c, lane);
                         }
@@ -1614,10 +1510,8 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                         for (u32 w = lane; w < 4u * nh; w += 32) S.aux[w] = 0u;
                         __syncwarp();
                     }
-                    u32 blo, bhi;
-                    const u32 c = boundary_cells_run<KIND>(S, P, a, nh, i0, min(hm.split, nh), bra, bla, brb, blb,
-                                                           blo, bhi, masks);
-                    if (c) combine<NFB>(S.part, resb, act, blo, bhi, c, lane);
+                    const u32 c = boundary_cells_run<KIND>(S, P, a, nh, i0, brun, blen, masks);
+                    if (c) combine<NFB>(S.part, resb, act, lane * blen, lane * blen + blen, c, lane);
                     if (masks && act)
                         a.bmask[i] = make_uint4(S.aux[4 * lane], S.aux[4 * lane + 1], S.aux[4 * lane + 2],
                                                 S.aux[4 * lane + 3]);
@@ -1634,7 +1528,6 @@ __device__ __forceinline__ void cell_pass_chunk(const DevParams& P, const TravAr
                     finish_row<KIND, BATCH>(P, a, i, res, resb, row_cnt, scene, dt, np_dt, red_max, red_speed,
                                             red_speed2);
             }
-            }   // units
         }
     }
 
@@ -1672,7 +1565,8 @@ __device__ __forceinline__ void reorder_cell_item(const float4* WCSPH_RESTRICT p
                                                   const DevState* st, u32 n, float cs, float4* WCSPH_RESTRICT pos_out,
                                                   float4* WCSPH_RESTRICT vel_out, u32* WCSPH_RESTRICT perm_out,
                                                   u64* WCSPH_RESTRICT ckey_out, u64* table, u32* cstart, u32* cend,
-                                                  u32 tmask, DevState* st_err, const u32* WCSPH_RESTRICT scene_in, u32 i) {
+                                                  u32 tmask, DevState* st_err, const u32* WCSPH_RESTRICT scene_in, u32 i,
+                                                  u32* units = nullptr, u32 unit_level = 0) {
     const u32 lane = threadIdx.x & 31u;
     const u32 sel = st->sort_sel[8];
     const u32* perm = sel == 0 ? nullptr : (sel == 1 ? v1 : v2);
@@ -1697,6 +1591,17 @@ __device__ __forceinline__ void reorder_cell_item(const float4* WCSPH_RESTRICT p
         const u32 s2 = guard_st(st_err, perm ? perm[i + 1] : i + 1, n);
         next = cell_key_of<BATCH>(pos_in[s2], cs, scene_in, s2);
     }
+    if (units) {   // list the blocks of 2^unit_level cells that start here, in any order
+        const u64 bm = block_mask<BATCH>(unit_level);
+        const bool first = valid && (i == 0 || ((pk ^ prev) & bm) != 0ull);
+        const u32 starts = __ballot_sync(FULL, first);
+        if (starts) {
+            u32 at = 0;
+            if (lane == 0) at = atomicAdd(&st_err->unit_count, static_cast<u32>(__popc(starts)));
+            at = __shfl_sync(FULL, at, 0);
+            if (first) units[at + __popc(starts & ((1u << lane) - 1u))] = i;
+        }
+    }
     if (!valid) return;
     // rebuild_n_search.cu:19-34: a run of equal cells starts where the key
     // changes and ends (non-inclusive) at the next change.
@@ -1715,3 +1620,5 @@ __device__ __forceinline__ void reorder_cell_item(const float4* WCSPH_RESTRICT p
 
 }  // namespace
 }  // namespace wcsph
+
+#include "density_blocks.cuh"

@@ -2,6 +2,7 @@
 #include "step_kernels.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 
 #include "step_device.cuh"
@@ -38,6 +39,15 @@ __global__ void __launch_bounds__(WPB * 32, KindCfg<KIND>::min_warps / WPB) cell
     if constexpr (KIND == PASS_SURFACE) surface_reduce<WPB>(a, dt, np_dt, red_max, red_speed, red_speed2);
 }
 
+
+// Density pass over blocks of 2^LEVEL cells (density_blocks.cuh).
+template <int LEVEL, bool BATCH>
+__global__ void __launch_bounds__(BlockCfg<LEVEL>::nt, BlockCfg<LEVEL>::min_blocks)
+density_block_kernel(const DevParams P, const TravArgs a) {
+    if (a.st->error_flags & ERR_LOOKBACK_TIMEOUT) return;   // no sorted state this step (reorder skipped)
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    density_units<BlockCfg<LEVEL>, BATCH>(P, a, *reinterpret_cast<BlockSmem<BlockCfg<LEVEL>>*>(dyn_smem));
+}
 
 // Resident warps per SM the register allocation of the list kernels must
 // allow (36 -> 56 registers, 44 -> 46, 48 -> 42). Both passes wait on
@@ -80,12 +90,13 @@ __global__ void reorder_cells_kernel(const float4* __restrict__ pos_in, const fl
                                      const DevState* st, u32 n, float cs, float4* __restrict__ pos_out,
                                      float4* __restrict__ vel_out, u32* __restrict__ perm_out,
                                      u64* __restrict__ ckey_out, u64* table, u32* cstart, u32* cend,
-                                     u32 tmask, DevState* st_err, const u32* __restrict__ scene_in) {
+                                     u32 tmask, DevState* st_err, const u32* __restrict__ scene_in,
+                                     u32* __restrict__ units, u32 unit_level) {
     // a sort whose look-back wait ran out left no permutation: keep the
     // previous sorted state and hash (every later pass returns at once too)
     if (st->error_flags & ERR_LOOKBACK_TIMEOUT) return;
     reorder_cell_item<BATCH>(pos_in, vel_in, v1, v2, st, n, cs, pos_out, vel_out, perm_out, ckey_out, table, cstart,
-                             cend, tmask, st_err, scene_in, blockIdx.x * blockDim.x + threadIdx.x);
+                             cend, tmask, st_err, scene_in, blockIdx.x * blockDim.x + threadIdx.x, units, unit_level);
 }
 
 __global__ void init_cfl_kernel(const float4* __restrict__ vel, u32 n, DevState* st) {
@@ -161,18 +172,18 @@ u32 pass_grid(u32 n, int wpb, u32 chunk) {
 void launch_reorder_cells(const float4* pos_in, const float4* vel_in, const u32* perm_src1, const u32* perm_src2,
                           const DevState* st, u32 n, float cs, float4* pos_out, float4* vel_out, u32* perm_out,
                           u64* ckey_out, u64* table, u32* cstart, u32* cend, u32 tmask, DevState* st_err,
-                          cudaStream_t stream, const u32* scene_in) {
+                          cudaStream_t stream, const u32* scene_in, u32* units, u32 unit_level) {
     if (n == 0) return;
     const u32 threads = 256;
     const u32 grid = (n + threads - 1) / threads;
     if (scene_in)
         reorder_cells_kernel<true><<<grid, threads, 0, stream>>>(pos_in, vel_in, perm_src1, perm_src2, st, n, cs,
                                                                  pos_out, vel_out, perm_out, ckey_out, table, cstart,
-                                                                 cend, tmask, st_err, scene_in);
+                                                                 cend, tmask, st_err, scene_in, units, unit_level);
     else
         reorder_cells_kernel<false><<<grid, threads, 0, stream>>>(pos_in, vel_in, perm_src1, perm_src2, st, n, cs,
                                                                   pos_out, vel_out, perm_out, ckey_out, table, cstart,
-                                                                  cend, tmask, st_err, nullptr);
+                                                                  cend, tmask, st_err, nullptr, units, unit_level);
 }
 
 template <int KIND, int WPB, bool BATCH>
@@ -195,11 +206,40 @@ static void launch_wpb(const DevParams& P, const TravArgs& a, cudaStream_t strea
     cell_pass_kernel<KIND, WPB, BATCH><<<grid, WPB * 32, bytes, stream>>>(P, a);
 }
 
+template <int LEVEL, bool BATCH>
+static void launch_density_blocks(const DevParams& P, const TravArgs& a, cudaStream_t stream) {
+    using C = BlockCfg<LEVEL>;
+    constexpr int kMaxDevices = 64;
+    static std::atomic<u32> resident[kMaxDevices];   // resident blocks of the device, 0 = not yet asked
+    int dev = 0;
+    cudaGetDevice(&dev);
+    u32 blocks = dev < kMaxDevices ? resident[dev].load() : 0u;
+    if (blocks == 0) {
+        int per_sm = 0, sms = 0;
+        cudaFuncSetAttribute(density_block_kernel<LEVEL, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(sizeof(BlockSmem<C>)));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, density_block_kernel<LEVEL, BATCH>, C::nt,
+                                                      sizeof(BlockSmem<C>));
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        blocks = static_cast<u32>(std::max(per_sm, 1) * std::max(sms, 1));
+        if (dev < kMaxDevices) resident[dev].store(blocks);
+    }
+    density_block_kernel<LEVEL, BATCH><<<std::min(blocks, a.n), C::nt, sizeof(BlockSmem<C>), stream>>>(P, a);
+}
+
 template <int KIND, bool BATCH>
 static void launch_kind(const DevParams& P, const TravArgs& a, cudaStream_t stream, int wpb) {
     const bool listed = (KIND == PASS_FORCE || KIND == PASS_SURFACE) && a.nbr != nullptr;
     const u32 grid = pass_grid(a.n, wpb, listed ? list_rows_per_warp(a.chunk) : a.chunk);
     if (grid == 0) return;
+    if constexpr (KIND == PASS_DENSITY) {
+        if (a.units) {
+            if (a.unit_level == 3u) launch_density_blocks<3, BATCH>(P, a, stream);
+            else if (a.unit_level == 6u) launch_density_blocks<6, BATCH>(P, a, stream);
+            else launch_density_blocks<5, BATCH>(P, a, stream);
+            return;
+        }
+    }
     switch (wpb) {
     case 2: launch_wpb<KIND, 2, BATCH>(P, a, stream, grid); break;
     case 8: launch_wpb<KIND, 8, BATCH>(P, a, stream, grid); break;

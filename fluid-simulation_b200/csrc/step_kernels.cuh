@@ -15,10 +15,12 @@
 //                   CFL max |v|^2 and metric reductions
 //                   (compute_non_pressure_accel.cu + update_positions.cu:14-68)
 //
-// Work decomposition (the density pass, and every pass when the lists are
-// off): one warp per chunk of 8, 16 or 32 particles of the sorted array
-// (small scenes use small chunks so that more warps run); for every cell
-// that starts inside the chunk, the warp looks
+// Work decomposition. With neighbour lists on and a neighbourhood one cell
+// deep, the density pass works on blocks of cells (density_blocks.cuh). With
+// the lists off, with two cells (cell size below 2h/3) and for the adjoint,
+// the passes take cells: one warp per chunk of 8, 16 or 32 particles of the
+// sorted array (small scenes use small chunks so that more warps run); for
+// every cell that starts inside the chunk, the warp looks
 // up the (2R+1)^3 neighbour cells once (lane-parallel hash probes) and
 // stages their particles (the candidates, in the reference's cell order)
 // into shared memory. The home particles are taken in blocks of up to 32.
@@ -28,9 +30,10 @@
 //                  candidate; rows padded to whole words), testing two
 //                  candidates per packed-FP32 step; phase 2 sums W over the
 //                  set bits. The matrix is kept row-major in the cell's
-//                  mask_words * n_home words of the mask buffer;
+//                  mask_words * n_home words of the mask buffer where a later
+//                  pass reads it;
 //   later passes   walk the set bits of that matrix (neighbours only).
-// With neighbour lists on (nbr != nullptr), the density pass also writes each
+// With neighbour lists on (nbr != nullptr), the density pass writes each
 // particle's neighbours, in candidate order, to its nbr_width list slots
 // (slot-major, so that a warp's rows read one slot coalesced), and the force
 // and surface passes no longer look at cells: lane k of a warp takes
@@ -84,10 +87,15 @@ struct TravArgs {
     // neighbour bitmasks
     u32* mask;
     u32 mask_words;           // words per particle (candidate cap = 32*mask_words)
-    u32 pair_cells;           // density with lists: x-pairs of cells share one traversal; the bit
-                              // matrix is then not kept (nothing reads it: the lists carry the sets)
+    u32 keep_matrix;          // the density pass stores its bit matrix (later passes walk it: lists off, or
+                              // the adjoint)
     u32 matrix_valid;         // neighbour export: the mask buffer holds the last density pass's matrix
     u32 chunk;                // sorted particles per warp chunk: 8, 16 or 32
+    // density units: first sorted particle of each Morton-aligned block of
+    // 2^unit_level cells (count in st->unit_count; nullptr: the density pass
+    // takes chunks of cells)
+    const u32* units;
+    u32 unit_level;
     // neighbour lists (nullptr: the force and surface passes walk the bit matrix)
     u32* nbr;                 // slot t of particle i at nbr[t * n + i], t < nbr_width, candidate order
     u32* nbr_cnt;             // per particle: neighbour count, or NBR_SPILL
@@ -141,7 +149,15 @@ void launch_reorder_cells(const float4* pos_in, const float4* vel_in, const u32*
                           const u32* perm_src2, const DevState* st, u32 n, float cs, float4* pos_out,
                           float4* vel_out, u32* perm_out, u64* ckey_out, u64* table, u32* cstart,
                           u32* cend, u32 tmask, DevState* st_err, cudaStream_t stream,
-                          const u32* scene_in = nullptr);
+                          const u32* scene_in = nullptr, u32* units = nullptr, u32 unit_level = 0);
+
+// Cells per density unit (BlockCfg), as a power of two. Larger units look up
+// and stage fewer cells per row (8, 4.5 and 3.4 candidates a row), smaller
+// ones give more thread blocks and a shorter last wave. Density pass in us at
+// levels 3 / 5 / 6: 33 k particles with walls 30 / 35 / 48, 79 k 53 / 65 / 80,
+// 393 k with walls 136 / 124 / 134, 0.7 M settled 246 / 260 / 251, 1 M
+// 254 / 226 / 208, 4 M 1092 / 1003 / 823.
+inline u32 unit_level(u32 n) { return n < (1u << 18) ? 3u : (n < (1u << 19) ? 5u : 6u); }
 
 void launch_pass(int kind, const DevParams& P, const TravArgs& a, cudaStream_t stream, int warps_per_block,
                  bool batch = false);
