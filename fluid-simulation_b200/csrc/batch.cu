@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "batch.cuh"
+#include "cluster_sort.cuh"
 #include "radix_sort.cuh"
 #include "step_kernels.cuh"
 
@@ -179,13 +180,7 @@ struct BatchSim {
     }
 
     void enqueue_step(float delta) {
-        WCSPH_CUDA(cudaMemsetAsync(table.ptr, 0xff, table.bytes(), stream));
-        keys_hist_kernel<<<std::min<u32>((n + 255) / 256, 1184), 256, 0, stream>>>(pos_a.ptr, n, dp.cell_size,
-                                                                                   keys[0].ptr, hist.ptr, scene_a.ptr);
-        SortBuffers sb{};
-        for (int i = 0; i < 3; ++i) { sb.keys[i] = keys[i].ptr; sb.vals[i] = vals[i].ptr; }
-        sb.hist = hist.ptr; sb.offsets = offs.ptr; sb.lookback = lookback.ptr; sb.capacity = n;
-        WCSPH_CUDA(enqueue_sort_passes(sb, n, st.ptr, stream));
+        if (!enqueue_small_sort()) enqueue_large_sort();
         launch_reorder_cells(pos_a.ptr, vel_a.ptr, vals[1].ptr, vals[2].ptr, st.ptr, n, dp.cell_size, pos_b.ptr,
                              vel_b.ptr, perm.ptr, ckey.ptr, table.ptr, cstart.ptr, cend.ptr, table_size - 1, st.ptr,
                              stream, scene_a.ptr, use_units() ? unit_buf() : nullptr, batch_unit_level(false));
@@ -193,6 +188,33 @@ struct BatchSim {
         launch_pass(PASS_DENSITY, dp, a, stream, 2, true);
         launch_pass(PASS_FORCE, dp, a, stream, 2, true);
         launch_pass(PASS_SURFACE, dp, a, stream, 2, true);
+    }
+
+    // Keys, sort and hash clear of a small ensemble in one launch (cluster_sort.cuh).
+    bool enqueue_small_sort() {
+        ClusterSortArgs c{};
+        c.pos = pos_a.ptr;
+        c.scene = scene_a.ptr;
+        c.n = n;
+        c.cs = dp.cell_size;
+        c.keys_out = keys[0].ptr;
+        c.perm = vals[1].ptr;
+        c.st = st.ptr;
+        c.table = table.ptr;
+        c.table_size = table_size;
+        bool launched = false;
+        WCSPH_CUDA(enqueue_cluster_sort(c, stream, &launched));
+        return launched;
+    }
+
+    void enqueue_large_sort() {
+        WCSPH_CUDA(cudaMemsetAsync(table.ptr, 0xff, table.bytes(), stream));
+        keys_hist_kernel<<<std::min<u32>((n + 255) / 256, 1184), 256, 0, stream>>>(pos_a.ptr, n, dp.cell_size,
+                                                                                   keys[0].ptr, hist.ptr, scene_a.ptr);
+        SortBuffers sb{};
+        for (int i = 0; i < 3; ++i) { sb.keys[i] = keys[i].ptr; sb.vals[i] = vals[i].ptr; }
+        sb.hist = hist.ptr; sb.offsets = offs.ptr; sb.lookback = lookback.ptr; sb.capacity = n;
+        WCSPH_CUDA(enqueue_sort_passes(sb, n, st.ptr, stream));
     }
 
     PersistentStep persistent_args(float delta, int steps) {

@@ -12,6 +12,7 @@ std::atomic<bool> g_sort_stall_test{false};
 }
 
 void set_sort_stall_test(bool on) { g_sort_stall_test.store(on); }
+bool sort_stall_test() { return g_sort_stall_test.load(); }
 
 
 __global__ void keys_hist_kernel(const float4* __restrict__ pos, u32 n, float cs,

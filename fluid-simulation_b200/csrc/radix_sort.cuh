@@ -87,5 +87,6 @@ cudaError_t enqueue_sort_passes(const SortBuffers& b, u32 n, DevState* st, cudaS
 // Error-path test hook: while on, sorts enqueued afterwards stall tile 0's
 // look-back flags and wait at most LB_SPIN_LIMIT_STALLED polls.
 void set_sort_stall_test(bool on);
+bool sort_stall_test();
 
 }  // namespace wcsph

@@ -2,6 +2,7 @@
 // parity field export. Reference orchestration: CUDASPHSimulator::update
 // (src/cuda/SPH/sph.cu:31-60) -> StepTuner::launch (step_tuner.cuh:259-295).
 #include "simulator.cuh"
+#include "cluster_sort.cuh"
 #include "render.cuh"
 
 #include <algorithm>
@@ -329,19 +330,40 @@ TravArgs CUDASPHSimulator::trav_args(float delta) {
     return a;
 }
 
-void CUDASPHSimulator::enqueue_search(bool keys_from_state) {
+void CUDASPHSimulator::enqueue_search() {
     NvtxRange r("wcsph sort + neighbourhood search");
     const u32 n = n_;
-    WCSPH_CUDA(cudaMemsetAsync(table_.ptr, 0xff, table_.bytes(), stream_));
-    if (keys_from_state) enqueue_keys();
-    SortBuffers sb{};
-    for (int i = 0; i < 3; ++i) { sb.keys[i] = keys_[i].ptr; sb.vals[i] = vals_[i].ptr; }
-    sb.keys[0] = ckeys_.ptr;   // the sort reads the compressed keys; keys_[0] keeps the field
-    sb.hist = hist_.ptr; sb.offsets = offsets_.ptr; sb.lookback = lookback_.ptr; sb.capacity = n;
-    WCSPH_CUDA(enqueue_sort_passes(sb, n, st_.ptr, stream_));
+    if (!enqueue_small_sort()) {
+        WCSPH_CUDA(cudaMemsetAsync(table_.ptr, 0xff, table_.bytes(), stream_));
+        enqueue_keys();
+        enqueue_sort();
+    }
     launch_reorder_cells(pos_a_.ptr, vel_a_.ptr, vals_[1].ptr, vals_[2].ptr, st_.ptr, n, dp_.cell_size, pos_b_.ptr,
                          vel_b_.ptr, perm_.ptr, ckey_.ptr, table_.ptr, cstart_.ptr, cend_.ptr, table_size_ - 1,
                          st_.ptr, stream_, nullptr, use_units() ? unit_buf() : nullptr, unit_level(n_));
+}
+
+bool CUDASPHSimulator::enqueue_small_sort() {
+    ClusterSortArgs c{};
+    c.pos = pos_a_.ptr;
+    c.n = n_;
+    c.cs = dp_.cell_size;
+    c.keys_out = keys_[0].ptr;
+    c.perm = vals_[1].ptr;
+    c.st = st_.ptr;
+    c.table = table_.ptr;
+    c.table_size = table_size_;
+    bool launched = false;
+    WCSPH_CUDA(enqueue_cluster_sort(c, stream_, &launched));
+    return launched;
+}
+
+void CUDASPHSimulator::enqueue_sort() {
+    SortBuffers sb{};
+    for (int i = 0; i < 3; ++i) { sb.keys[i] = keys_[i].ptr; sb.vals[i] = vals_[i].ptr; }
+    sb.keys[0] = ckeys_.ptr;   // the sort reads the compressed keys; keys_[0] keeps the field
+    sb.hist = hist_.ptr; sb.offsets = offsets_.ptr; sb.lookback = lookback_.ptr; sb.capacity = n_;
+    WCSPH_CUDA(enqueue_sort_passes(sb, n_, st_.ptr, stream_));
 }
 
 void CUDASPHSimulator::enqueue_keys() {
@@ -366,7 +388,7 @@ TravArgs CUDASPHSimulator::fixed_args(float dt) {
 }
 
 void CUDASPHSimulator::enqueue_fixed_step(float dt) {
-    enqueue_search(true);
+    enqueue_search();
     const TravArgs a = fixed_args(dt);
     launch_pass(PASS_DENSITY, dp_, a, stream_, cfg_.warps_density);
     launch_pass(PASS_FORCE, dp_, a, stream_, cfg_.warps_force);
@@ -375,7 +397,7 @@ void CUDASPHSimulator::enqueue_fixed_step(float dt) {
 
 void CUDASPHSimulator::enqueue_step(float delta) {
     NvtxRange r("wcsph step");
-    enqueue_search(true);
+    enqueue_search();
     const TravArgs a = trav_args(delta);
     {
         NvtxRange rd("wcsph density pass");
@@ -392,8 +414,9 @@ void CUDASPHSimulator::enqueue_step(float delta) {
 }
 
 int CUDASPHSimulator::launches_per_step() const {
-    // keys_bounds + compressed_keys_hist + sort_plan + 8 onesweep + reorder_cells + 3 cell passes
-    return 2 + 1 + SORT_DIGITS + 1 + 3;
+    // small scenes: cluster sort, else keys_bounds + compressed_keys_hist + sort_plan + 8 onesweep;
+    // then reorder_cells and the three passes
+    return (n_ <= CLUSTER_SORT_MAX ? 1 : 2 + 1 + SORT_DIGITS) + 1 + 3;
 }
 
 void CUDASPHSimulator::invalidate_graph() {
@@ -667,14 +690,16 @@ int CUDASPHSimulator::kernel_timings(const char** names, float* ms, int cap) {
     const float delta = graph_valid_ ? graph_delta_ : params_.max_time_step;
     const u32 n = n_;
     WCSPH_CUDA(cudaEventRecord(ev[0], stream_));
-    WCSPH_CUDA(cudaMemsetAsync(table_.ptr, 0xff, table_.bytes(), stream_));
-    enqueue_keys();
+    // small scenes: the cluster sort computes the keys itself (keys_hist 0)
     WCSPH_CUDA(cudaEventRecord(ev[1], stream_));
-    SortBuffers sb{};
-    for (int i = 0; i < 3; ++i) { sb.keys[i] = keys_[i].ptr; sb.vals[i] = vals_[i].ptr; }
-    sb.keys[0] = ckeys_.ptr;
-    sb.hist = hist_.ptr; sb.offsets = offsets_.ptr; sb.lookback = lookback_.ptr; sb.capacity = n;
-    WCSPH_CUDA(enqueue_sort_passes(sb, n, st_.ptr, stream_));
+    const bool small = enqueue_small_sort();
+    if (!small) {
+        WCSPH_CUDA(cudaEventRecord(ev[0], stream_));
+        WCSPH_CUDA(cudaMemsetAsync(table_.ptr, 0xff, table_.bytes(), stream_));
+        enqueue_keys();
+        WCSPH_CUDA(cudaEventRecord(ev[1], stream_));
+        enqueue_sort();
+    }
     WCSPH_CUDA(cudaEventRecord(ev[2], stream_));
     launch_reorder_cells(pos_a_.ptr, vel_a_.ptr, vals_[1].ptr, vals_[2].ptr, st_.ptr, n, dp_.cell_size, pos_b_.ptr,
                          vel_b_.ptr, perm_.ptr, ckey_.ptr, table_.ptr, cstart_.ptr, cend_.ptr, table_size_ - 1,

@@ -178,7 +178,12 @@ public:
     // Enqueues one step without graph capture (also used inside capture).
     void enqueue_step(float delta);
     // Enqueues sort + neighbourhood search of one step on the current state.
-    void enqueue_search(bool keys_from_state);
+    void enqueue_search();
+    // Keys, sort and hash clear of small scenes in one launch (cluster_sort.cuh);
+    // false: nothing enqueued, enqueue_keys and enqueue_sort apply.
+    bool enqueue_small_sort();
+    // The onesweep sort of the compressed keys.
+    void enqueue_sort();
     // Traversal arguments with a fixed time step (CFL off): dt_p = dt.
     TravArgs fixed_args(float dt);
     // One step with a fixed time step (the differentiable rollout's forward).

@@ -214,10 +214,11 @@ static void launch_density_blocks(const DevParams& P, const TravArgs& a, cudaStr
     int dev = 0;
     cudaGetDevice(&dev);
     u32 blocks = dev < kMaxDevices ? resident[dev].load() : 0u;
+    // on every call: the attribute belongs to the current context
+    cudaFuncSetAttribute(density_block_kernel<LEVEL, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         static_cast<int>(sizeof(BlockSmem<C>)));
     if (blocks == 0) {
         int per_sm = 0, sms = 0;
-        cudaFuncSetAttribute(density_block_kernel<LEVEL, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(sizeof(BlockSmem<C>)));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, density_block_kernel<LEVEL, BATCH>, C::nt,
                                                       sizeof(BlockSmem<C>));
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
