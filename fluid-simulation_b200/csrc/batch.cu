@@ -124,10 +124,8 @@ struct BatchSim {
 
     // density units: see CUDASPHSimulator::use_units
     bool use_units() const { return nbr_width > 0 && dp.range == 1; }
-    // The persistent kernel's 256-thread blocks take units of 4x4x2 cells at
-    // least (12 / 64 / 256 scenes, ms per step at levels 3, 5, 6: 0.571 / 1.81 /
-    // 6.80, 0.455 / 1.28 / 4.49, 0.480 / 1.27 / 4.33).
-    u32 batch_unit_level(bool persistent) const { return persistent ? std::max(unit_level(n), 5u) : unit_level(n); }
+    // (the persistent kernel's buffers hold units of 4x4x2 cells)
+    u32 batch_unit_level(bool persistent) const { return persistent ? 5u : unit_level(n); }
     u32* unit_buf() { return reinterpret_cast<u32*>(keys[1].ptr); }
 
     // persistent: the persistent kernel's traversal phases (16 particles per

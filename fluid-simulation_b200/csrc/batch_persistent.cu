@@ -77,10 +77,16 @@ __device__ __forceinline__ bool grid_barrier(u32* bar, DevState* st, u32 limit) 
     return s_go != 0u;
 }
 
-// Density units in the persistent kernel: 256-thread blocks, the largest capacity.
+// Density units in the persistent kernel: 4x4x2 cells by 256 threads. What the
+// three resident blocks take as shared memory is missing as L1 in the list
+// phases, so the buffers are small (256 scenes, ms per step: 3.56 with 1792
+// candidates and 8 words, 3.62 with 2048 and 10, 4.37 with 3072 and 12 for
+// 4x4x4 cells; four blocks of 64 registers 3.44, but 0.42 against 0.37 at 12
+// scenes).
 struct PersistentBlock {
-    static constexpr int nt = PTHREADS, cap = 3072, words = 12;
+    static constexpr int nt = PTHREADS, cap = 1792, words = 8;
 };
+constexpr u32 PERSISTENT_BLOCKS = 3;   // resident blocks per SM (80 registers)
 
 size_t persistent_smem(const TravArgs& a) {
     const u32 cap = a.mask_words * 32u;
@@ -96,7 +102,10 @@ size_t persistent_smem(const TravArgs& a) {
     return b;
 }
 
-__global__ void __launch_bounds__(PTHREADS, 3) persistent_ensemble_kernel(const PersistentStep ps) {
+// UNITS: the density phase takes blocks of cells (a.units); a kernel of its own,
+// because the code of both kinds of density phase together spills.
+template <bool UNITS>
+__global__ void __launch_bounds__(PTHREADS, PERSISTENT_BLOCKS) persistent_ensemble_kernel(const PersistentStep ps) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ u32 s_tile;
     __shared__ u32 s_active[SORT_DIGITS];
@@ -148,7 +157,7 @@ __global__ void __launch_bounds__(PTHREADS, 3) persistent_ensemble_kernel(const 
                                     const_cast<u32*>(a.units), a.unit_level);
         if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;
         const u32 nchunks = (n + a.chunk - 1) / a.chunk;
-        if (a.units) {
+        if constexpr (UNITS) {
             density_units<PersistentBlock, true>(P, a, *reinterpret_cast<BlockSmem<PersistentBlock>*>(smem));
         } else {
             const WarpView<PASS_DENSITY> S = warp_view<PASS_DENSITY>(a, smem, warp);
@@ -157,12 +166,11 @@ __global__ void __launch_bounds__(PTHREADS, 3) persistent_ensemble_kernel(const 
                     cell_pass_chunk<PASS_DENSITY, true>(P, a, S, c, 0.f, 0.f, rm, rs, rs2);
         }
         if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;
-        const u32 rows = list_rows_per_warp(a.chunk);
-        const u32 ngroups = (n + rows - 1) / rows;
-        if (a.nbr) {
+        const u32 ngroups = (n + LIST_ROWS - 1) / LIST_ROWS;
+        if (UNITS || a.nbr) {
             for (u32 g0 = claim(ps.barrier + WORK_FORCE); g0 < ngroups; g0 = claim(ps.barrier + WORK_FORCE))
                 for (u32 g = g0; g < min(g0 + CLAIM, ngroups); ++g)
-                    list_rows<PASS_FORCE, true, 1>(P, a, g * rows, min(rows, n - g * rows), 0.f, 0.f, rm, rs, rs2);
+                    list_rows<PASS_FORCE, true, 2>(P, a, g * LIST_ROWS, min(LIST_ROWS, n - g * LIST_ROWS), 0.f, 0.f, rm, rs, rs2);
         } else {
             const WarpView<PASS_FORCE> S = warp_view<PASS_FORCE>(a, smem, warp);
             for (u32 c0 = claim(ps.barrier + WORK_FORCE); c0 < nchunks; c0 = claim(ps.barrier + WORK_FORCE))
@@ -171,10 +179,10 @@ __global__ void __launch_bounds__(PTHREADS, 3) persistent_ensemble_kernel(const 
         }
         if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;
         const float dt = cfl_time_step(a, P);   // fixed step: the bounds alone decide
-        if (a.nbr) {
+        if (UNITS || a.nbr) {
             for (u32 g0 = claim(ps.barrier + WORK_SURFACE); g0 < ngroups; g0 = claim(ps.barrier + WORK_SURFACE))
                 for (u32 g = g0; g < min(g0 + CLAIM, ngroups); ++g)
-                    list_rows<PASS_SURFACE, true, 2>(P, a, g * rows, min(rows, n - g * rows), dt, np_dt, rm, rs, rs2);
+                    list_rows<PASS_SURFACE, true, 2>(P, a, g * LIST_ROWS, min(LIST_ROWS, n - g * LIST_ROWS), dt, np_dt, rm, rs, rs2);
         } else {
             const WarpView<PASS_SURFACE> S = warp_view<PASS_SURFACE>(a, smem, warp);
             for (u32 c0 = claim(ps.barrier + WORK_SURFACE); c0 < nchunks; c0 = claim(ps.barrier + WORK_SURFACE))
@@ -189,10 +197,11 @@ __global__ void __launch_bounds__(PTHREADS, 3) persistent_ensemble_kernel(const 
 
 void persistent_grid(const TravArgs& a, int device, u32* blocks, size_t* smem) {
     const size_t bytes = persistent_smem(a);
-    WCSPH_CUDA(cudaFuncSetAttribute(persistent_ensemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const auto fn = a.units ? persistent_ensemble_kernel<true> : persistent_ensemble_kernel<false>;
+    WCSPH_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(bytes)));
     int per_sm = 0, sms = 0;
-    WCSPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_ensemble_kernel, PTHREADS, bytes));
+    WCSPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PTHREADS, bytes));
     WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     if (per_sm < 1) throw Error(WCSPH_ERR_NOT_SUPPORTED, "persistent ensemble kernel does not fit on an SM");
     *blocks = static_cast<u32>(per_sm * sms);
@@ -210,7 +219,7 @@ void launch_persistent(const PersistentStep& ps, u32 blocks, size_t smem, cudaSt
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    WCSPH_CUDA(cudaLaunchKernelEx(&cfg, persistent_ensemble_kernel, ps));
+    WCSPH_CUDA(cudaLaunchKernelEx(&cfg, ps.a.units ? persistent_ensemble_kernel<true> : persistent_ensemble_kernel<false>, ps));
 }
 
 }  // namespace wcsph

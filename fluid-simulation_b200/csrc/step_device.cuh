@@ -1080,7 +1080,8 @@ __device__ __forceinline__ void spill_row(const DevParams& P, const TravArgs& a,
 // Boundary sums of one row (particle i, home data H): the 3x3x3 boundary
 // cells around its own cell in x, y, z nesting order, as for_boundary_neighbors
 // (common.cuh:153-178) visits them, one particle after the other.
-template <int KIND, bool BATCH>
+// DEPTH: marked candidates in flight while one is summed.
+template <int KIND, bool BATCH, int DEPTH = 1>
 __device__ __forceinline__ void boundary_row(const DevParams& P, const TravArgs& a, const HomeData& H, u32 scene,
                                              float* resb, u32 i) {
     const int3 c = cell_of(H.x, P.h);
@@ -1091,12 +1092,30 @@ __device__ __forceinline__ void boundary_row(const DevParams& P, const TravArgs&
             // the density pass of this step marked the candidates within h
             // (same positions, same predicate): visit those, in run order
             const uint4 mk = ro_ld(a.bmask + i);
-            const u32 words[4] = {mk.x, mk.y, mk.z, mk.w};
+            u64 now = (static_cast<u64>(mk.y) << 32) | mk.x, later = (static_cast<u64>(mk.w) << 32) | mk.z;
+            const u32 hits = __popc(mk.x) + __popc(mk.y) + __popc(mk.z) + __popc(mk.w);
+            u32 off = t;
+            auto next = [&]() -> float4 {   // the next marked candidate
+                if (now == 0ull) {
+                    now = later;
+                    later = 0ull;
+                    off = t + 64u;
+                }
+                const u32 bit = static_cast<u32>(__ffsll(static_cast<long long>(now))) - 1u;
+                now &= now - 1ull;
+                return ro_ld(a.bcx + guard(a, off + bit, a.bcx_n));
+            };
+            float4 xb[DEPTH + 1];   // DEPTH candidates in flight while one is summed
 #pragma unroll
-            for (u32 w = 0; w < 4; ++w) {
-                for (u32 bits = words[w]; bits; bits &= bits - 1) {
-                    const float4 xb = ro_ld(a.bcx + guard(a, t + 32u * w + (__ffs(bits) - 1), a.bcx_n));
-                    boundary_pair_m<KIND>(resb, H, xb.w, xb, dist2(H.x, xb), P);
+            for (int u = 0; u <= DEPTH; ++u)
+                if (static_cast<u32>(u) < hits) xb[u] = next();
+            for (u32 h = 0; h < hits; h += DEPTH + 1) {
+#pragma unroll
+                for (int u = 0; u <= DEPTH; ++u) {
+                    if (h + u < hits) {
+                        boundary_pair_m<KIND>(resb, H, xb[u].w, xb[u], dist2(H.x, xb[u]), P);
+                        if (h + u + DEPTH + 1 < hits) xb[u] = next();
+                    }
                 }
             }
             return;
@@ -1130,12 +1149,8 @@ __device__ __forceinline__ void boundary_row(const DevParams& P, const TravArgs&
 // particles [i0, i0 + nh) of its chunk, whatever their cells; lane k sums
 // row k's list in order (the reference's per-particle order), so a row's
 // sums do not depend on which particles share its warp.
-// DEPTH: neighbour records in flight per lane while a pair is summed (1, or
-// 2 where the registers are there anyway: the persistent ensemble kernel
-// runs at the density pass's register budget, with fewer resident warps than
-// the list kernels; its surface phase gains from the second record in flight,
-// its force phase does not).
-template <int KIND, bool BATCH, int DEPTH = 1>
+// DEPTH: neighbours summed together, with the next DEPTH in flight.
+template <int KIND, bool BATCH, int DEPTH>
 __device__ __forceinline__ void list_rows(const DevParams& P, const TravArgs& a, u32 i0, u32 nh, float dt,
                                           float np_dt, float& red_max, float& red_speed, float& red_speed2) {
     using C = KindCfg<KIND>;
@@ -1165,46 +1180,41 @@ __device__ __forceinline__ void list_rows(const DevParams& P, const TravArgs& a,
     if (act) {
         const HomeData H = load_home<KIND>(a, i);
         if (!spill && cnt > 0) {
-            // slot t of row i at nbr[t * n + i]; the next neighbour's records
-            // and the index after it are in flight while a pair is summed
+            // Slot t of row i at nbr[t * n + i]. Groups of DEPTH neighbours: the
+            // next group's records and the indices of the one after are in
+            // flight while a group is summed, in list order; a group's pairs
+            // are independent up to their sums. Past the end the last index is
+            // read again.
             const size_t stride = a.n;
-            if constexpr (DEPTH == 1) {
-                const u32* lst = a.nbr + i + stride;
-                Nbr d = fetch_j<KIND>(a, ro_ld(a.nbr + i));
-                u32 jn = cnt > 1 ? ro_ld(lst) : 0u;
-                lst += stride;
-                for (u32 t = 0; t < cnt; ++t) {
-                    Nbr dn = d;
-                    if (t + 1 < cnt) dn = fetch_j<KIND>(a, jn);
-                    if (t + 2 < cnt) {
-                        jn = ro_ld(lst);
-                        lst += stride;
-                    }
-                    fluid_pair<KIND>(res, H, d, dist2(H.x, d.x), P, a);
-                    d = dn;
-                }
-            } else {
-                const u32* lst = a.nbr + i;
-                Nbr d0 = fetch_j<KIND>(a, ro_ld(lst));
-                Nbr d1 = d0;
-                if (cnt > 1) d1 = fetch_j<KIND>(a, ro_ld(lst + stride));
-                u32 jn = cnt > 2 ? ro_ld(lst + 2 * stride) : 0u;
-                lst += 3 * stride;
-                for (u32 t = 0; t < cnt; ++t) {
-                    Nbr d2 = d1;
-                    if (t + 2 < cnt) d2 = fetch_j<KIND>(a, jn);
-                    if (t + 3 < cnt) {
-                        jn = ro_ld(lst);
-                        lst += stride;
-                    }
-                    fluid_pair<KIND>(res, H, d0, dist2(H.x, d0.x), P, a);
-                    d0 = d1;
-                    d1 = d2;
-                }
+            constexpr u32 N = DEPTH;
+            const u32* lst = a.nbr + i;
+            auto index = [&](u32 t) { return ro_ld(lst + min(t, cnt - 1u) * stride); };
+            Nbr d[N];
+            u32 jn[N];
+#pragma unroll
+            for (u32 u = 0; u < N; ++u) jn[u] = index(u);
+#pragma unroll
+            for (u32 u = 0; u < N; ++u) d[u] = fetch_j<KIND>(a, jn[u]);
+#pragma unroll
+            for (u32 u = 0; u < N; ++u) jn[u] = index(N + u);
+            u32 t = 0;
+            for (; t + N <= cnt; t += N) {
+                Nbr dn[N];
+#pragma unroll
+                for (u32 u = 0; u < N; ++u) dn[u] = fetch_j<KIND>(a, jn[u]);
+#pragma unroll
+                for (u32 u = 0; u < N; ++u) jn[u] = index(t + 2u * N + u);
+#pragma unroll
+                for (u32 u = 0; u < N; ++u) fluid_pair<KIND>(res, H, d[u], dist2(H.x, d[u].x), P, a);
+#pragma unroll
+                for (u32 u = 0; u < N; ++u) d[u] = dn[u];
             }
+#pragma unroll
+            for (u32 u = 0; u + 1u < N; ++u)
+                if (t + u < cnt) fluid_pair<KIND>(res, H, d[u], dist2(H.x, d[u].x), P, a);
         }
         if constexpr (C::boundary) {
-            if (a.nb > 0) boundary_row<KIND, BATCH>(P, a, H, scene, resb, i);
+            if (a.nb > 0) boundary_row<KIND, BATCH, (DEPTH > 2 ? DEPTH : 1)>(P, a, H, scene, resb, i);
         }
     }
     if (act) finish_row<KIND, BATCH>(P, a, i, res, resb, 0u, scene, dt, np_dt, red_max, red_speed, red_speed2);
@@ -1545,9 +1555,8 @@ __device__ __forceinline__ WarpView<KIND> warp_view(const TravArgs& a, unsigned 
     return S;
 }
 
-// Particles per warp of the list kernels: one per lane, except for small
-// scenes (density chunks of 8), which keep 8 so that more warps run.
-__host__ __device__ inline u32 list_rows_per_warp(u32 chunk) { return chunk == 8u ? 8u : 32u; }
+// Particles per warp of the list kernels: one per lane.
+constexpr u32 LIST_ROWS = 32;
 
 template <bool BATCH>
 __device__ __forceinline__ u64 cell_key_of(float4 p, float cs, const u32* scene_in, u32 src) {

@@ -49,23 +49,28 @@ density_block_kernel(const DevParams P, const TravArgs a) {
     density_units<BlockCfg<LEVEL>, BATCH>(P, a, *reinterpret_cast<BlockSmem<BlockCfg<LEVEL>>*>(dyn_smem));
 }
 
-// Resident warps per SM the register allocation of the list kernels must
-// allow (36 -> 56 registers, 44 -> 46, 48 -> 42). Both passes wait on
-// neighbour gathers, so resident warps pay while spills stay small: the
-// force pass fits 56 registers (36 warps; at 48 it spills), the single-scene
-// surface pass 40 (50 warps with two-warp blocks, against 40 at the 47 it
-// takes when allowed 48). The batched passes carry the scene lookups: 56
-// registers cost the force pass 4 bytes of spills and still gain (ensemble
-// step 5.34 -> 5.27 ms); the batched surface pass runs at a 44-warp cap.
-template <int KIND, bool BATCH>
+// Neighbours summed together (list_rows' DEPTH) and resident warps per SM the
+// register allocation of the list kernels must allow (36 -> 56 registers, 32 ->
+// 64). Both passes wait on neighbour gathers. Above 2^18 particles two
+// neighbours at a time, with the next two in flight, gain more than the warps
+// they cost: force at 36 warps 141 -> 121 us at 1 M particles, 497 -> 430 at 4 M
+// (28 warps 126 / 461, 40 warps spill: 166 / 629; three at a time 136 / 505),
+// surface at 32 warps 155 -> 150 and 143 -> 138 (0.7 M settled). Smaller scenes
+// leave the SMs a few warps each, so three at a time are summed with 128
+// registers to spare: force / surface 27 / 27 -> 20 / 17 us at 33 k particles
+// with walls, 55 / 55 -> 28 / 26 at 79 k (half of that by full warps: these
+// scenes took 8 rows per warp before).
+constexpr u32 LIST_SMALL = 1u << 18;
+template <int KIND, bool SMALL>
 struct ListCfg {
-    static constexpr int min_warps = KIND == PASS_FORCE ? 36 : (BATCH ? 44 : 48);
+    static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : 32);
+    static constexpr int depth = SMALL ? 3 : 2;
 };
 
 // Force / surface pass over the neighbour lists written by the density pass.
-template <int KIND, int WPB, bool BATCH>
-__global__ void __launch_bounds__(WPB * 32, ListCfg<KIND, BATCH>::min_warps / WPB) list_pass_kernel(const DevParams P,
-                                                                                          const TravArgs a) {
+template <int KIND, int WPB, bool BATCH, bool SMALL>
+__global__ void __launch_bounds__(WPB * 32, ListCfg<KIND, SMALL>::min_warps / WPB)
+list_pass_kernel(const DevParams P, const TravArgs a) {
     if (a.st->error_flags & ERR_LOOKBACK_TIMEOUT) return;   // no sorted state this step (reorder skipped)
     const u32 lane = lane_id();
     const u32 warp = threadIdx.x >> 5;
@@ -77,10 +82,10 @@ __global__ void __launch_bounds__(WPB * 32, ListCfg<KIND, BATCH>::min_warps / WP
         np_dt = a.delta < a.np_max_dt ? a.delta : a.np_max_dt;
     }
     float red_max = 0.f, red_speed = 0.f, red_speed2 = 0.f;
-    const u32 rows = list_rows_per_warp(a.chunk);
-    const u32 base = (blockIdx.x * WPB + warp) * rows;
+    const u32 base = (blockIdx.x * WPB + warp) * LIST_ROWS;
     if (base < a.n)
-        list_rows<KIND, BATCH>(P, a, base, min(rows, a.n - base), dt, np_dt, red_max, red_speed, red_speed2);
+        list_rows<KIND, BATCH, ListCfg<KIND, SMALL>::depth>(P, a, base, min(LIST_ROWS, a.n - base), dt, np_dt, red_max,
+                                                            red_speed, red_speed2);
     if constexpr (KIND == PASS_SURFACE) surface_reduce<WPB>(a, dt, np_dt, red_max, red_speed, red_speed2);
 }
 
@@ -191,7 +196,8 @@ static void launch_wpb(const DevParams& P, const TravArgs& a, cudaStream_t strea
     // per-warp candidate staging sized by the bit-matrix capacity 32 * mask_words
     if constexpr (KIND == PASS_FORCE || KIND == PASS_SURFACE) {
         if (a.nbr) {   // the list kernels use no shared memory (all of it serves as L1)
-            list_pass_kernel<KIND, WPB, BATCH><<<grid, WPB * 32, 0, stream>>>(P, a);
+            if (a.n < LIST_SMALL) list_pass_kernel<KIND, WPB, BATCH, true><<<grid, WPB * 32, 0, stream>>>(P, a);
+            else list_pass_kernel<KIND, WPB, BATCH, false><<<grid, WPB * 32, 0, stream>>>(P, a);
             return;
         }
     }
@@ -231,7 +237,7 @@ static void launch_density_blocks(const DevParams& P, const TravArgs& a, cudaStr
 template <int KIND, bool BATCH>
 static void launch_kind(const DevParams& P, const TravArgs& a, cudaStream_t stream, int wpb) {
     const bool listed = (KIND == PASS_FORCE || KIND == PASS_SURFACE) && a.nbr != nullptr;
-    const u32 grid = pass_grid(a.n, wpb, listed ? list_rows_per_warp(a.chunk) : a.chunk);
+    const u32 grid = pass_grid(a.n, wpb, listed ? LIST_ROWS : a.chunk);
     if (grid == 0) return;
     if constexpr (KIND == PASS_DENSITY) {
         if (a.units) {
