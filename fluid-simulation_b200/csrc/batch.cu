@@ -184,8 +184,8 @@ struct BatchSim {
                              stream, scene_a.ptr, use_units() ? unit_buf() : nullptr, batch_unit_level(false));
         const TravArgs a = args(delta);
         launch_pass(PASS_DENSITY, dp, a, stream, 2, true);
-        launch_pass(PASS_FORCE, dp, a, stream, 2, true);
-        launch_pass(PASS_SURFACE, dp, a, stream, 2, true);
+        launch_pass(PASS_FORCE, dp, a, stream, list_warps(PASS_FORCE, n), true);
+        launch_pass(PASS_SURFACE, dp, a, stream, list_warps(PASS_SURFACE, n), true);
     }
 
     // Keys, sort and hash clear of a small ensemble in one launch (cluster_sort.cuh).

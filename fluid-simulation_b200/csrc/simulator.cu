@@ -125,6 +125,8 @@ CUDASPHSimulator::CUDASPHSimulator(const wcsph_params& params, const wcsph_scene
     cfg_.table_size_mult = params_.table_size_mult;
     n_ = scene.fluid_n;
     nb_ = scene.boundary_n;
+    cfg_.warps_force = list_warps(PASS_FORCE, n_);
+    cfg_.warps_surface = list_warps(PASS_SURFACE, n_);
     init_pos_.assign(scene.fluid_pos, scene.fluid_pos + 4ull * n_);
 
     allocate();

@@ -99,8 +99,8 @@ float metric_mass(const wcsph_params& p);
 // Tunable launch configuration of the step (the autotuner's search space).
 struct StepConfig {
     int warps_density = 2;
-    int warps_force = 4;
-    int warps_surface = 2;
+    int warps_force = 4;        // by scene size at creation (list_warps)
+    int warps_surface = 8;
     int mask_words = 12;        // neighbour bit-matrix words per particle (cap = 32*words)
     int chunk = 0;              // sorted particles per warp: 8, 16, 32; 0 = by scene size
     int nbr_width = 64;         // neighbour-list slots per particle; 0 = walk the bit matrix

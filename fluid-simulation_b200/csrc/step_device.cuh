@@ -14,6 +14,8 @@
 #pragma once
 #include <climits>
 
+#include <cuda/atomic>
+
 #include "step_kernels.cuh"
 
 #ifndef WCSPH_COHERENT_LOADS
@@ -1220,6 +1222,14 @@ __device__ __forceinline__ void list_rows(const DevParams& P, const TravArgs& a,
     if (act) finish_row<KIND, BATCH>(P, a, i, res, resb, 0u, scene, dt, np_dt, red_max, red_speed, red_speed2);
 }
 
+// Counts an arrival after the caller's earlier writes (release). A full fence
+// (__threadfence) would also drop the SM's L1 contents at every warp's end,
+// which the other warps' gathers still use; only the last arriver, which reads
+// the others' partials, acquires.
+__device__ __forceinline__ u32 arrive(u32* counter) {
+    return cuda::atomic_ref<u32, cuda::thread_scope_device>(*counter).fetch_add(1u, cuda::memory_order_release);
+}
+
 // Surface pass: CFL max |v|^2 and the metric sums without block barriers:
 // warp partials -> groups of 32 warps -> whole grid; each level is finished
 // by its last arriving warp and summed in index order (deterministic). The
@@ -1245,11 +1255,10 @@ __device__ __forceinline__ void surface_reduce(const TravArgs& a, float dt, floa
         a.block_partials[2 * gw] = red_speed;
         a.block_partials[2 * gw + 1] = red_speed2;
         atomicMax(&a.st->vmax2_bits[a.st->parity ^ 1u], __float_as_uint(red_max));
-        __threadfence();
-        last = atomicAdd(a.group_done + group, 1u) == gsize - 1 ? 1u : 0u;
+        last = arrive(a.group_done + group) == gsize - 1 ? 1u : 0u;
     }
     if (__shfl_sync(FULL, last, 0)) {
-        __threadfence();
+        cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
         const u32 w = (group << 5) + lane;
         double s1 = lane < gsize ? static_cast<double>(__ldcg(a.block_partials + 2 * w)) : 0.0;
         double s2 = lane < gsize ? static_cast<double>(__ldcg(a.block_partials + 2 * w + 1)) : 0.0;
@@ -1262,11 +1271,10 @@ __device__ __forceinline__ void surface_reduce(const TravArgs& a, float dt, floa
             a.group_partials[2 * group] = s1;
             a.group_partials[2 * group + 1] = s2;
             a.group_done[group] = 0u;
-            __threadfence();
-            top = atomicAdd(&a.st->blocks_done, 1u) == ngroups - 1 ? 1u : 0u;
+            top = arrive(&a.st->blocks_done) == ngroups - 1 ? 1u : 0u;
         }
         if (__shfl_sync(FULL, top, 0)) {
-            __threadfence();
+            cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
             double t1 = 0.0, t2 = 0.0;
             for (u32 g = lane; g < ngroups; g += 32) {
                 t1 += __ldcg(a.group_partials + 2 * g);

@@ -50,21 +50,22 @@ density_block_kernel(const DevParams P, const TravArgs a) {
 }
 
 // Neighbours summed together (list_rows' DEPTH) and resident warps per SM the
-// register allocation of the list kernels must allow (36 -> 56 registers, 32 ->
-// 64). Both passes wait on neighbour gathers. Above 2^18 particles two
-// neighbours at a time, with the next two in flight, gain more than the warps
-// they cost: force at 36 warps 141 -> 121 us at 1 M particles, 497 -> 430 at 4 M
-// (28 warps 126 / 461, 40 warps spill: 166 / 629; three at a time 136 / 505),
-// surface at 32 warps 155 -> 150 and 143 -> 138 (0.7 M settled). Smaller scenes
-// leave the SMs a few warps each, so three at a time are summed with 128
-// registers to spare: force / surface 27 / 27 -> 20 / 17 us at 33 k particles
-// with walls, 55 / 55 -> 28 / 26 at 79 k (half of that by full warps: these
-// scenes took 8 rows per warp before).
-constexpr u32 LIST_SMALL = 1u << 18;
+// register allocation of the list kernels must allow (36 -> 56 registers, 48 ->
+// 40). Both passes wait on neighbour gathers.
+// Above 2^18 particles the force pass sums two neighbours at a time, with the
+// next two in flight, and gains more than the warps it costs: 1 M particles
+// 141 -> 121 us, 4 M 497 -> 430 (28 warps 126 / 461, 40 warps spill: 166 / 629,
+// three at a time 136 / 505). The surface pass keeps one at a time, all the
+// warps that fit and 8-warp blocks: 1 M 139 us, 4 M 474 (two at a time at 32
+// warps 143 / 516; 2-warp blocks 141 / 502).
+// Smaller scenes leave the SMs a few warps each, so three at a time are summed
+// with 128 registers to spare: force / surface 27 / 27 -> 20 / 16 us at 33 k
+// particles with walls, 55 / 55 -> 27 / 25 at 79 k (half of that by full warps:
+// these scenes took 8 rows per warp before).
 template <int KIND, bool SMALL>
 struct ListCfg {
-    static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : 32);
-    static constexpr int depth = SMALL ? 3 : 2;
+    static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : 48);
+    static constexpr int depth = SMALL ? 3 : (KIND == PASS_FORCE ? 2 : 1);
 };
 
 // Force / surface pass over the neighbour lists written by the density pass.

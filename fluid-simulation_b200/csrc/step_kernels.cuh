@@ -151,6 +151,12 @@ void launch_reorder_cells(const float4* pos_in, const float4* vel_in, const u32*
                           u32* cend, u32 tmask, DevState* st_err, cudaStream_t stream,
                           const u32* scene_in = nullptr, u32* units = nullptr, u32 unit_level = 0);
 
+// Below this many particles the list passes run their few-warps-per-SM variant
+// (ListCfg), best in 2-warp blocks; above, the force pass takes 4-warp blocks
+// and the surface pass 8-warp blocks.
+constexpr u32 LIST_SMALL = 1u << 18;
+inline int list_warps(int kind, u32 n) { return n < LIST_SMALL ? 2 : (kind == 1 ? 4 : 8); }
+
 // Cells per density unit (BlockCfg), as a power of two. Larger units look up
 // and stage fewer cells per row (8, 4.5 and 3.4 candidates a row), smaller
 // ones give more thread blocks and a shorter last wave. Density pass in us at
