@@ -69,16 +69,32 @@ __device__ __forceinline__ u32 range_cells(const TravArgs& a) {
     return d * d * d;
 }
 
+// Four slots of the cell hash (a 32-byte sector; tables have a power of two of
+// at least 64 slots).
+__device__ __forceinline__ void load_slots(const u64* p, u64* k) {
+    asm("ld.global" WCSPH_RO_QUAL ".v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(k[0]), "=l"(k[1]), "=l"(k[2]), "=l"(k[3])
+        : "l"(p));
+}
+
 // Linear-probed lookup of a packed cell key (find_cell_in_table,
 // common.cuh:89-102), with the loads of this file's flavour.
 template <bool BATCH = false>
 __device__ __forceinline__ u32 find_slot(const u64* WCSPH_RESTRICT table, u32 tmask, u64 pk) {
+    // four slots (one sector) at a time: chains of neighbouring cells are long
+    // enough for a dependent load per slot to show
     u32 t = static_cast<u32>(slot_hash<BATCH>(pk) & tmask);
-    for (u32 j = 0; j <= tmask; ++j) {
-        const u64 k = ro_ld(table + t);
-        if (k == EMPTY_HASH) return EMPTY_CELL;
-        if (k == pk) return t;
-        t = (t + 1) & tmask;
+    for (u32 j = 0; j <= tmask + 4u; j += 4u) {   // the first sector twice: from t on, then its start
+        const u32 base = t & ~3u;
+        u64 k[4];
+        load_slots(table + base, k);
+#pragma unroll
+        for (u32 q = 0; q < 4u; ++q) {
+            if (base + q < t) continue;
+            if (k[q] == EMPTY_HASH) return EMPTY_CELL;
+            if (k[q] == pk) return base + q;
+        }
+        t = (base + 4u) & tmask;
     }
     return EMPTY_CELL;
 }
@@ -1573,9 +1589,36 @@ __device__ __forceinline__ u64 cell_key_of(float4 p, float cs, const u32* scene_
     else return pack_cell(c);
 }
 
+// hash_insert four slots at a time: plain loads find the cell or the first free
+// slot, and only a free one costs an atomic.
+template <bool BATCH>
+__device__ __forceinline__ u32 insert_slot(u64* table, u32 tmask, u64 pk) {
+    u32 t = static_cast<u32>(slot_hash<BATCH>(pk) & tmask);
+    for (u32 j = 0; j <= tmask + 4u; j += 4u) {
+        const u32 base = t & ~3u;
+        u64 k[4];
+        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(k[0]), "=l"(k[1]) : "l"(table + base));
+        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(k[2]), "=l"(k[3]) : "l"(table + base + 2u));
+        for (u32 q = t - base; q < 4u; ++q) {
+            const u64 seen = q < 2u ? (q == 0u ? k[0] : k[1]) : (q == 2u ? k[2] : k[3]);
+            if (seen == pk) return base + q;
+            if (seen == EMPTY_HASH) {
+                const u64 old = atomicCAS(table + base + q, EMPTY_HASH, pk);
+                if (old == EMPTY_HASH || old == pk) return base + q;
+            }
+        }
+        t = (base + 4u) & tmask;
+    }
+    return EMPTY_CELL;
+}
+
 // Reorder + hash build for sorted index i (gather pos/vel into sorted order,
 // cell keys, run starts/ends into the hash; rebuild_n_search.cu:19-34). All 32
 // lanes of a warp must call it together (i >= n for the idle ones).
+// Bound by the latency of its dependent accesses (index, gather, hash): taking
+// the outer lanes' second gather, the probe chains' slots and the run ends'
+// second probe out of that chain gave 1 M particles 42 -> 33 us, 4 M 143 -> 119,
+// the 27 k droplet, whose cells crowd in the hash, 22 -> 17.
 template <bool BATCH>
 __device__ __forceinline__ void reorder_cell_item(const float4* WCSPH_RESTRICT pos_in, const float4* WCSPH_RESTRICT vel_in,
                                                   const u32* WCSPH_RESTRICT v1, const u32* WCSPH_RESTRICT v2,
@@ -1588,47 +1631,57 @@ __device__ __forceinline__ void reorder_cell_item(const float4* WCSPH_RESTRICT p
     const u32 sel = st->sort_sel[8];
     const u32* perm = sel == 0 ? nullptr : (sel == 1 ? v1 : v2);
     const bool valid = i < n;
+    // the outer lanes also fetch the particle beyond the warp's end, with the
+    // warp's own loads
+    const u32 e = lane == 0 ? i - 1u : i + 1u;
+    const bool edge = valid && ((lane == 0 && i > 0) || (lane == 31 && i + 1 < n));
+    const u32 src = valid ? guard_st(st_err, perm ? perm[i] : i, n) : 0u;
+    const u32 src2 = edge ? guard_st(st_err, perm ? perm[e] : e, n) : 0u;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), p2 = p, vel = p;
+    if (valid) p = pos_in[src];
+    if (edge) p2 = pos_in[src2];
+    if (valid && vel_out) vel = vel_in[src];
     u64 pk = 0;
     if (valid) {
-        const u32 src = guard_st(st_err, perm ? perm[i] : i, n);
-        const float4 p = pos_in[src];
         pos_out[i] = p;
-        if (vel_out) vel_out[i] = vel_in[src];
+        if (vel_out) vel_out[i] = vel;
         perm_out[i] = src;
         pk = cell_key_of<BATCH>(p, cs, scene_in, src);
         ckey_out[i] = pk;
     }
     u64 prev = __shfl_up_sync(FULL, pk, 1);
     u64 next = __shfl_down_sync(FULL, pk, 1);
-    if (valid && lane == 0 && i > 0) {
-        const u32 s2 = guard_st(st_err, perm ? perm[i - 1] : i - 1, n);
-        prev = cell_key_of<BATCH>(pos_in[s2], cs, scene_in, s2);
+    if (edge) {
+        const u64 k2 = cell_key_of<BATCH>(p2, cs, scene_in, src2);
+        if (lane == 0) prev = k2;
+        else next = k2;
     }
-    if (valid && lane == 31 && i + 1 < n) {
-        const u32 s2 = guard_st(st_err, perm ? perm[i + 1] : i + 1, n);
-        next = cell_key_of<BATCH>(pos_in[s2], cs, scene_in, s2);
-    }
+    // rebuild_n_search.cu:19-34: a run of equal cells starts where the key
+    // changes and ends (non-inclusive) at the next change.
+    const bool first = valid && (i == 0 || pk != prev);
+    const bool last = valid && (i == n - 1 || pk != next);
     if (units) {   // list the blocks of 2^unit_level cells that start here, in any order
         const u64 bm = block_mask<BATCH>(unit_level);
-        const bool first = valid && (i == 0 || ((pk ^ prev) & bm) != 0ull);
-        const u32 starts = __ballot_sync(FULL, first);
+        const bool opens = valid && (i == 0 || ((pk ^ prev) & bm) != 0ull);
+        const u32 starts = __ballot_sync(FULL, opens);
         if (starts) {
             u32 at = 0;
             if (lane == 0) at = atomicAdd(&st_err->unit_count, static_cast<u32>(__popc(starts)));
             at = __shfl_sync(FULL, at, 0);
-            if (first) units[at + __popc(starts & ((1u << lane) - 1u))] = i;
+            if (opens) units[at + __popc(starts & ((1u << lane) - 1u))] = i;
         }
     }
-    if (!valid) return;
-    // rebuild_n_search.cu:19-34: a run of equal cells starts where the key
-    // changes and ends (non-inclusive) at the next change.
-    if (i == 0 || pk != prev) {
-        const u32 slot = hash_insert<BATCH>(table, tmask, pk);
+    u32 slot = EMPTY_CELL;
+    if (first) {
+        slot = insert_slot<BATCH>(table, tmask, pk);
         if (slot == EMPTY_CELL) atomicOr(&st_err->error_flags, ERR_HASH_FULL);
         else cstart[slot] = i;
     }
-    if (i == n - 1 || pk != next) {
-        const u32 slot = hash_insert<BATCH>(table, tmask, pk);
+    // the end of a run that starts in this warp takes the slot its start found
+    const u32 before = __ballot_sync(FULL, first) & (FULL >> (31u - lane));
+    const u32 from = __shfl_sync(FULL, slot, before ? 31 - __clz(static_cast<int>(before)) : 0);
+    if (last) {
+        slot = before ? from : insert_slot<BATCH>(table, tmask, pk);
         if (slot == EMPTY_CELL) atomicOr(&st_err->error_flags, ERR_HASH_FULL);
         else cend[slot] = i + 1;
     }
