@@ -4,8 +4,8 @@
 // A unit of work is a Morton-aligned block of cells (2x2x2, 4x4x2 or 4x4x4:
 // its particles are contiguous in sorted order) and one thread block of NT
 // threads. The unit
-//   1. counts its particles (rows) and looks up the cells of the block and of
-//      the layer around it (64, 144 or 216), one thread per cell;
+//   1. looks up the cells of the block and of the layer around it (64, 144 or
+//      216), one lane per cell; the block's own cells add up to its rows;
 //   2. stages their particles (the candidates) in shared memory, cells in the
 //      x, y, z nesting order, as x / y / z / particle-index arrays;
 //   3. lets every lane take one row. The 27 cells around the row's cell are 9
@@ -25,13 +25,14 @@
 // What bounds it (1 M particles, 4x4x4 cells): instruction issue (141 M warp
 // instructions, 61 % of the cycles issue) and the shared-memory data pipe
 // (75 % busy: a 128-bit load costs three wavefronts for a warp's four or five
-// cells, a walked hit four loads of four). Of its 208 us, look-ups and counts
-// take about 35 (latency), staging 18, the tests 85, the walk 61, the epilogue
-// 18. The pass it replaced gave a warp the two cells of an x-pair (36 looked-up
-// cells and 18 staged candidates per row, where a row here pays for 3.4), split
-// their hits over the lanes and wrote the lists one scattered word at a time:
-// 349 M warp instructions, 460 us (4 M particles 2055 -> 823 us, 0.7 M settled
-// 434 -> 251, 33 k with walls 51 -> 30).
+// cells, a walked hit four loads of four). Of 208 us, look-ups took about 35
+// (latency; 203 since warps that are done look up for the next unit), staging
+// 18, the tests 85, the walk 61, the epilogue 18. The pass it replaced gave a
+// warp the two cells of an x-pair (36 looked-up cells and 18 staged candidates
+// per row, where a row here pays for 3.4), split their hits over the lanes and
+// wrote the lists one scattered word at a time: 349 M warp instructions, 460 us
+// (4 M particles 2055 -> 830 us, 0.7 M settled 434 -> 258, 33 k with walls
+// 51 -> 30).
 #pragma once
 
 namespace wcsph {
@@ -65,9 +66,15 @@ struct BlockSmem {
     u32 j[C::cap];
     u32 word[C::words * C::nt];
     unsigned short wbase[C::words * C::nt];
-    u32 rstart[BLOCK_CELLS];
-    u32 rpref[BLOCK_CELLS + 4];
-    u32 next;   // the unit claimed next
+    // cells of the running unit and of the next one: first particle, and the
+    // count, then exclusive prefix (+ total)
+    u32 rstart[2][BLOCK_CELLS];
+    u32 rpref[2][BLOCK_CELLS + 4];
+    u32 start[2];      // first row of the unit
+    u64 id[2];         // its block key
+    u32 rows[2];       // its particles
+    u32 next;          // the unit claimed next
+    u32 chunk;         // look-up chunks handed out
 };
 
 // Density of row i's boundary particles (cell size h cells, one lane): its
@@ -152,8 +159,8 @@ __device__ __forceinline__ u32 density_direct_row(const DevParams& P, const Trav
 // row's own candidate index. Returns the neighbour count.
 template <class C>
 __device__ __forceinline__ u32 density_staged_row(const DevParams& P, const TravArgs& a, BlockSmem<C>& S, u32 i,
-                                                  float4 xi, u32 seg0, u32 Dy, u32 Dz, u32 selfm, bool act, float& t3,
-                                                  float& u3) {
+                                                  float4 xi, const u32* rpref, u32 seg0, u32 Dy, u32 Dz, u32 selfm,
+                                                  bool act, float& t3, float& u3) {
     const float2 nx = make_float2(-xi.x, -xi.x), ny = make_float2(-xi.y, -xi.y), nz = make_float2(-xi.z, -xi.z);
     const float lim = -__uint_as_float(__float_as_uint(P.h2) + 1u);   // minus the float after h2
     const float2 nlim = make_float2(lim, lim);
@@ -170,8 +177,8 @@ __device__ __forceinline__ u32 density_staged_row(const DevParams& P, const Trav
         while (seg < 9u && k < static_cast<u32>(C::words)) {
             if (!open) {
                 const u32 c = seg0 + ((seg / 3u) * Dy + seg % 3u) * Dz;
-                s0 = S.rpref[c];
-                e0 = S.rpref[c + 3u];
+                s0 = rpref[c];
+                e0 = rpref[c + 3u];
                 b = s0 & ~3u;
             }
             if (b < e0) {
@@ -238,155 +245,188 @@ __device__ __forceinline__ u32 density_staged_row(const DevParams& P, const Trav
     return hits;
 }
 
-// The particles of the block that starts at sorted index `start`, by the whole
-// thread block.
-template <class C, bool BATCH>
-__device__ __forceinline__ void density_unit(const DevParams& P, const TravArgs& a, BlockSmem<C>& S, u32 start) {
-    const u32 tid = threadIdx.x;
-    const u32 lane = tid & 31u;
-    const u32 n = a.n;
-    u32 level = a.unit_level;
-    const u64 unit_mask = block_mask<BATCH>(level);
-    u32 i0 = start;
-    const u64 unit_id = a.ckey[i0] & unit_mask;
-    for (;;) {
-        const u64 pk0 = a.ckey[i0];
-        const u64 mask = block_mask<BATCH>(level);
-        const u64 id = pk0 & mask;
-        u32 ux, uy, uz, scene;
+// A block of 2^level cells with its surrounding layer.
+template <bool BATCH>
+struct BlockGrid {
+    u32 ox, oy, oz, scene;   // first cell of the layer
+    u32 Dx, Dy, Dz;
+    __device__ __forceinline__ BlockGrid(u64 id, u32 level) {
+        u32 ux, uy, uz;
         decode_cell<BATCH>(id, ux, uy, uz, scene);
-        const u32 lx = (level + 2u) / 3u, ly = (level + 1u) / 3u, lz = level / 3u;
-        const u32 ox = ux - 1u, oy = uy - 1u, oz = uz - 1u;   // first cell of the surrounding layer
-        const u32 Dx = (1u << lx) + 2u, Dy = (1u << ly) + 2u, Dz = (1u << lz) + 2u;
-        const u32 ncell = Dx * Dy * Dz;
-        // keys of the first rows, in flight during the lookups
-        u64 rk[3];
-#pragma unroll
-        for (u32 k = 0; k < 3u; ++k) {
-            const u32 i = i0 + k * C::nt + tid;
-            rk[k] = i < n ? a.ckey[i] : ~id;
-        }
-        // cells of the block and its layer: start and count
-        for (u32 q = tid; q < ncell; q += C::nt) {
-            const u32 x = q / (Dy * Dz), y = (q / Dz) % Dy, z = q % Dz;
+        ox = ux - 1u; oy = uy - 1u; oz = uz - 1u;
+        Dx = (1u << ((level + 2u) / 3u)) + 2u;
+        Dy = (1u << ((level + 1u) / 3u)) + 2u;
+        Dz = (1u << (level / 3u)) + 2u;
+    }
+    __device__ __forceinline__ u32 cells() const { return Dx * Dy * Dz; }
+};
+
+// Looks up the cells of block `id` into buffer b, 32 at a time: warps take
+// chunks from S.chunk (zeroed before, as S.rows[b]). The block's own cells
+// add up to its rows.
+template <class C, bool BATCH>
+__device__ __forceinline__ void density_lookup(const TravArgs& a, BlockSmem<C>& S, u32 b, u64 id, u32 level) {
+    const u32 lane = lane_id();
+    const BlockGrid<BATCH> G(id, level);
+    const u32 ncell = G.cells();
+    for (;;) {
+        u32 c = 0;
+        if (lane == 0) c = atomicAdd(&S.chunk, 1u);
+        c = __shfl_sync(FULL, c, 0);
+        if (c * 32u >= ncell) break;
+        const u32 q = c * 32u + lane;
+        u32 mine = 0;
+        if (q < ncell) {
+            const u32 x = q / (G.Dy * G.Dz), y = (q / G.Dz) % G.Dy, z = q % G.Dz;
             u64 pk;
-            if constexpr (BATCH) pk = pack_cell_batch(scene, ox + x, oy + y, oz + z);
-            else pk = pack_cell(ox + x, oy + y, oz + z);
-            const u32 slot = find_slot<BATCH>(a.fluid.table, a.fluid.tmask, pk);
+            if constexpr (BATCH) pk = pack_cell_batch(G.scene, G.ox + x, G.oy + y, G.oz + z);
+            else pk = pack_cell(G.ox + x, G.oy + y, G.oz + z);
+            const u32 slot = find_slot_wide<BATCH>(a.fluid.table, a.fluid.tmask, pk);
             u32 s = 0, cnt = 0;
             if (slot != EMPTY_CELL) {
                 s = ro_ld(a.fluid.cstart + slot);
                 const u32 e = ro_ld(a.fluid.cend + slot);
                 cnt = e > s ? e - s : 0u;
             }
-            S.rstart[q] = s;
-            S.rpref[q] = cnt;
+            S.rstart[b][q] = s;
+            S.rpref[b][q] = cnt;
+            if (x - 1u < G.Dx - 2u && y - 1u < G.Dy - 2u && z - 1u < G.Dz - 2u) mine = cnt;
         }
-        // rows of the block: the run of equal block keys from i0 on
-        u32 rows = 0;
-        for (u32 base = i0;;) {
-            bool more = true;
-#pragma unroll
-            for (u32 k = 0; k < 3u; ++k) {
-                if (!more) continue;
-                const u32 c = static_cast<u32>(__syncthreads_count((rk[k] & mask) == id));
-                rows += c;
-                more = c == static_cast<u32>(C::nt);
-            }
-            if (!more) break;
-            base += 3u * C::nt;
-#pragma unroll
-            for (u32 k = 0; k < 3u; ++k) {
-                const u32 i = base + k * C::nt + tid;
-                rk[k] = i < n ? a.ckey[i] : ~id;
-            }
-        }
-        // exclusive prefix of the counts (the barrier above made them visible)
-        if (tid < 32u) {
-            u32 run = 0;
-            for (u32 base = 0; base < ncell; base += 32u) {
-                const u32 q = base + lane;
-                const u32 c = q < ncell ? S.rpref[q] : 0u;
-                const u32 incl = warp_incl_scan(c);
-                if (q < ncell) S.rpref[q] = run + incl - c;
-                run += __shfl_sync(FULL, incl, 31);
-            }
-            if (lane == 0) S.rpref[ncell] = run;
-        }
-        __syncthreads();
-        const u32 M = S.rpref[ncell];
-        if (M > static_cast<u32>(C::cap) && level > 0u) {   // too dense: smaller blocks, same thread block
-            --level;
-            __syncthreads();
-            continue;
-        }
-        const bool staged = M <= static_cast<u32>(C::cap);
-        if (staged) {
-            // eight lanes per cell: a cell's particles are contiguous
-            for (u32 q = tid >> 3; q < ncell; q += C::nt / 8) {
-                const u32 s = S.rstart[q], m0 = S.rpref[q], cnt = S.rpref[q + 1u] - m0;
-                for (u32 t = tid & 7u; t < cnt; t += 8u) {
-                    const u32 j = guard(a, s + t, n);
-                    const float4 p = ro_ld(a.pos + j);
-                    const u32 m = guard(a, m0 + t, C::cap);
-                    S.x[m] = p.x;
-                    S.y[m] = p.y;
-                    S.z[m] = p.z;
-                    S.j[m] = j;
-                }
-            }
-        }
-        __syncthreads();
-        for (u32 r0 = tid & ~31u; r0 < rows; r0 += C::nt) {
-            const u32 r = r0 + lane;
-            const bool act = r < rows;
-            const u32 i = i0 + (act ? r : 0u);
-            const u64 pk = a.ckey[i];
-            const float4 xi = ro_ld(a.pos + guard(a, i, n));
-            float t3 = 0.f, u3 = 0.f;
-            u32 hits = 0;
-            if (staged) {
-                u32 cx, cy, cz, sc;
-                decode_cell<BATCH>(pk, cx, cy, cz, sc);
-                cx -= ox; cy -= oy; cz -= oz;   // 1 .. D - 2 per axis
-                const u32 cell = guard(a, (cx * Dy + cy) * Dz + cz, ncell);
-                const u32 s = S.rstart[cell], m0 = S.rpref[cell];
-                const u32 selfm = i - s < S.rpref[cell + 1u] - m0 ? m0 + (i - s) : 0xFFFF0000u;
-                hits = density_staged_row<C>(P, a, S, i, xi, cell - (Dy + 1u) * Dz - 1u, Dy, Dz, selfm, act, t3, u3);
-            } else if (act) {
-                hits = density_direct_row<BATCH>(P, a, i, pk, xi, t3, u3);
-            }
-            if (act) {
-                const float res[1] = {__fmaf_rn(2.f, t3, -u3)};
-                float resb[1] = {0.f};
-                if (a.nb > 0) density_boundary_row<BATCH>(P, a, xi, scene, i, resb);
-                float r_max = 0.f, r_s = 0.f, r_s2 = 0.f;
-                finish_row<PASS_DENSITY, BATCH>(P, a, i, res, resb, hits <= a.nbr_width ? hits : NBR_SPILL, scene, 0.f,
-                                                0.f, r_max, r_s, r_s2);
-            }
-        }
-        if (level == a.unit_level) return;
-        i0 += rows;
-        if (i0 >= n || (a.ckey[i0] & unit_mask) != unit_id) return;   // the same for every thread
-        __syncthreads();
+        mine = __reduce_add_sync(FULL, mine);
+        if (lane == 0 && mine) atomicAdd(&S.rows[b], mine);
     }
 }
 
-// Units of the whole array, claimed from a device counter (the next claim is
-// in flight while a unit is worked on). The list and both counters are
-// rebuilt by the sort plan and the reorder of every step.
+// Units of the whole array, by thread blocks that claim them from a device
+// counter (the list and both counters are rebuilt by the sort plan and the
+// reorder of every step). Warps that have finished their rows of a unit look
+// the next one's cells up while the others still work: their dependent
+// loads (list, key, hash, range) took 34 of 208 us at 1 M particles (256 scenes
+// per stage 3.12 -> 2.93 ms a step, 1 M 209 -> 203 us).
 template <class C, bool BATCH>
 __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs& a, BlockSmem<C>& S) {
+    const u32 tid = threadIdx.x;
+    const u32 lane = tid & 31u;
+    const u32 n = a.n;
     const u32 count = *reinterpret_cast<const volatile u32*>(&a.st->unit_count);
-    u32 u = blockIdx.x;   // the first claim of every block is its own index
-    while (u < count) {
-        u32 nxt = 0;
-        if (threadIdx.x == 0) nxt = atomicAdd(&a.st->unit_next, 1u) + gridDim.x;
-        density_unit<C, BATCH>(P, a, S, guard(a, a.units[u], a.n));
-        __syncthreads();
-        if (threadIdx.x == 0) S.next = nxt;
-        __syncthreads();
-        u = S.next;
+    const u64 unit_mask = block_mask<BATCH>(a.unit_level);
+    // the first claim of every block is its own index
+    if (blockIdx.x >= count) return;
+    auto lookup_unit = [&](u32 u, u32 b) {
+        const u32 start = guard(a, a.units[u], n);
+        const u64 id = a.ckey[start] & unit_mask;
+        if (tid == 0) {
+            S.start[b] = start;
+            S.id[b] = id;
+        }
+        density_lookup<C, BATCH>(a, S, b, id, a.unit_level);
+    };
+    if (tid == 0) {
+        S.chunk = 0u;
+        S.rows[0] = 0u;
+    }
+    __syncthreads();
+    lookup_unit(blockIdx.x, 0u);
+    for (u32 b = 0;; b ^= 1u) {
+        u32 claimed = 0;
+        if (tid == 0) claimed = atomicAdd(&a.st->unit_next, 1u) + gridDim.x;
+        __syncthreads();   // the unit's look-ups, and the last rows of the one before
+        u32 level = a.unit_level;
+        u32 i0 = S.start[b];
+        u64 id = S.id[b];
+        for (;;) {
+            const BlockGrid<BATCH> G(id, level);
+            const u32 ncell = G.cells();
+            // exclusive prefix of the counts
+            if (tid < 32u) {
+                u32 run = 0;
+                for (u32 base = 0; base < ncell; base += 32u) {
+                    const u32 q = base + lane;
+                    const u32 c = q < ncell ? S.rpref[b][q] : 0u;
+                    const u32 incl = warp_incl_scan(c);
+                    if (q < ncell) S.rpref[b][q] = run + incl - c;
+                    run += __shfl_sync(FULL, incl, 31);
+                }
+                if (lane == 0) {
+                    S.rpref[b][ncell] = run;
+                    S.next = claimed;
+                    S.chunk = 0u;
+                    S.rows[b ^ 1u] = 0u;
+                }
+            }
+            __syncthreads();
+            const u32 M = S.rpref[b][ncell];
+            const u32 rows = min(S.rows[b], n - i0);
+            const bool split = M > static_cast<u32>(C::cap) && level > 0u;   // too dense: smaller blocks
+            const bool staged = M <= static_cast<u32>(C::cap);
+            if (staged) {
+                // eight lanes per cell: a cell's particles are contiguous
+                for (u32 q = tid >> 3; q < ncell; q += C::nt / 8) {
+                    const u32 s = S.rstart[b][q], m0 = S.rpref[b][q], cnt = S.rpref[b][q + 1u] - m0;
+                    for (u32 t = tid & 7u; t < cnt; t += 8u) {
+                        const u32 j = guard(a, s + t, n);
+                        const float4 p = ro_ld(a.pos + j);
+                        const u32 m = guard(a, m0 + t, C::cap);
+                        S.x[m] = p.x;
+                        S.y[m] = p.y;
+                        S.z[m] = p.z;
+                        S.j[m] = j;
+                    }
+                }
+            }
+            __syncthreads();
+            if (!split) {
+                for (u32 r0 = tid & ~31u; r0 < rows; r0 += C::nt) {
+                    const u32 r = r0 + lane;
+                    const bool act = r < rows;
+                    const u32 i = i0 + (act ? r : 0u);
+                    const u64 pk = a.ckey[i];
+                    const float4 xi = ro_ld(a.pos + guard(a, i, n));
+                    float t3 = 0.f, u3 = 0.f;
+                    u32 hits = 0;
+                    if (staged) {
+                        u32 cx, cy, cz, sc;
+                        decode_cell<BATCH>(pk, cx, cy, cz, sc);
+                        cx -= G.ox; cy -= G.oy; cz -= G.oz;   // 1 .. D - 2 per axis
+                        const bool in = cx - 1u < G.Dx - 2u && cy - 1u < G.Dy - 2u && cz - 1u < G.Dz - 2u;
+                        const u32 ring = (G.Dy + 1u) * G.Dz + 1u;   // from the first of the 27 cells to their middle
+                        const u32 cell = in ? (cx * G.Dy + cy) * G.Dz + cz : ring;
+                        const u32 s = S.rstart[b][cell], m0 = S.rpref[b][cell];
+                        const u32 selfm = i - s < S.rpref[b][cell + 1u] - m0 ? m0 + (i - s) : 0xFFFF0000u;
+                        hits = density_staged_row<C>(P, a, S, i, xi, S.rpref[b], cell - ring, G.Dy, G.Dz, selfm,
+                                                     act && in, t3, u3);
+                    } else if (act) {
+                        hits = density_direct_row<BATCH>(P, a, i, pk, xi, t3, u3);
+                    }
+                    if (act) {
+                        const float res[1] = {__fmaf_rn(2.f, t3, -u3)};
+                        float resb[1] = {0.f};
+                        if (a.nb > 0) density_boundary_row<BATCH>(P, a, xi, G.scene, i, resb);
+                        float r_max = 0.f, r_s = 0.f, r_s2 = 0.f;
+                        finish_row<PASS_DENSITY, BATCH>(P, a, i, res, resb, hits <= a.nbr_width ? hits : NBR_SPILL,
+                                                        G.scene, 0.f, 0.f, r_max, r_s, r_s2);
+                    }
+                }
+                if (level == a.unit_level) break;
+                i0 += rows;
+                if (rows == 0u || i0 >= n || (a.ckey[i0] & unit_mask) != S.id[b]) break;   // the same for every thread
+            } else {
+                --level;
+            }
+            // the next part of a split unit
+            id = a.ckey[i0] & block_mask<BATCH>(level);
+            __syncthreads();
+            if (tid == 0) {
+                S.chunk = 0u;
+                S.rows[b] = 0u;
+            }
+            __syncthreads();
+            density_lookup<C, BATCH>(a, S, b, id, level);
+            __syncthreads();
+        }
+        const u32 next = S.next;
+        if (next >= count) return;
+        lookup_unit(next, b ^ 1u);
     }
 }
 
