@@ -191,22 +191,22 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
     const u32 n = n_;
     const int nck = steps / every + 1;
     A.steps = steps; A.every = every; A.dt = dt;
-    A.ck_pos.alloc(static_cast<size_t>(nck) * n); A.ck_vel.alloc(static_cast<size_t>(nck) * n);
-    A.ck_ids.alloc(static_cast<size_t>(nck) * n);
+    // workspaces are kept from one rollout to the next (an optimisation calls this
+    // once per iteration with the same sizes)
+    A.ck_pos.ensure(static_cast<size_t>(nck) * n); A.ck_vel.ensure(static_cast<size_t>(nck) * n);
+    A.ck_ids.ensure(static_cast<size_t>(nck) * n);
     if (static_cast<int>(A.seg.size()) != every) A.seg = std::vector<StepSet>(every);
     for (StepSet& b : A.seg) {
-        if (b.pos_b.count != n) {
-            b.pos_b.alloc(n); b.vel_b.alloc(n); b.ap.alloc(n); b.vlap.alloc(n);
-            b.perm.alloc(n); b.ckey.alloc(n); b.rho.alloc(n); b.prs.alloc(n);
-        }
-        if (b.table.count != table_size_) { b.table.alloc(table_size_); b.cstart.alloc(table_size_); b.cend.alloc(table_size_); }
-        if (b.mask.count != mask_.count) b.mask.alloc(mask_.count);
+        b.pos_b.ensure(n); b.vel_b.ensure(n); b.ap.ensure(n); b.vlap.ensure(n);
+        b.perm.ensure(n); b.ckey.ensure(n); b.rho.ensure(n); b.prs.ensure(n);
+        b.table.ensure(table_size_); b.cstart.ensure(table_size_); b.cend.ensure(table_size_);
+        b.mask.ensure(mask_.count);
     }
-    A.ids_a.alloc(n); A.ids_b.alloc(n);
-    A.target.alloc(n); A.final_pos.alloc(n); A.final_vel.alloc(n);
-    A.xbar.alloc(n); A.vbar.alloc(n); A.xbar_s.alloc(n); A.vbar_s.alloc(n); A.abar.alloc(n); A.w.alloc(n);
-    A.rhobar.alloc(n);
-    A.accum.alloc(3);
+    A.ids_a.ensure(n); A.ids_b.ensure(n);
+    A.target.ensure(n); A.final_pos.ensure(n); A.final_vel.ensure(n);
+    A.xbar.ensure(n); A.vbar.ensure(n); A.xbar_s.ensure(n); A.vbar_s.ensure(n); A.abar.ensure(n); A.w.ensure(n);
+    A.rhobar.ensure(n);
+    A.accum.ensure(3);
     WCSPH_CUDA(cudaMemcpyAsync(A.target.ptr, target_host, sizeof(float4) * n, cudaMemcpyHostToDevice, stream_));
     invalidate_graph();
     iota_kernel<<<blocks(n), 256, 0, stream_>>>(A.ids_a.ptr, n);

@@ -148,6 +148,7 @@ CUDASPHSimulator::~CUDASPHSimulator() {
         if (e) cudaEventDestroy(e);
     if (box_pinned_) cudaFreeHost(box_pinned_);
     if (metrics_pinned_) cudaFreeHost(metrics_pinned_);
+    if (flags_pinned_) cudaFreeHost(flags_pinned_);
     tuner_.reset();
 }
 
@@ -263,7 +264,6 @@ void CUDASPHSimulator::init_boundary(const float* bpos_host) {
 
 void CUDASPHSimulator::upload_state(const float* pos, const float* vel) {
     WCSPH_CUDA(cudaMemcpyAsync(pos_a_.ptr, pos, sizeof(float4) * n_, cudaMemcpyHostToDevice, stream_));
-    WCSPH_CUDA(cudaMemcpyAsync(pos_b_.ptr, pos, sizeof(float4) * n_, cudaMemcpyHostToDevice, stream_));
     if (vel) WCSPH_CUDA(cudaMemcpyAsync(vel_a_.ptr, vel, sizeof(float4) * n_, cudaMemcpyHostToDevice, stream_));
     else WCSPH_CUDA(cudaMemsetAsync(vel_a_.ptr, 0, sizeof(float4) * n_, stream_));
     // fresh CFL maximum of the new state
@@ -277,6 +277,10 @@ void CUDASPHSimulator::upload_state(const float* pos, const float* vel) {
 void CUDASPHSimulator::check_device_errors() {
     u32 flags = 0;
     WCSPH_CUDA(cudaMemcpy(&flags, &st_.ptr->error_flags, sizeof(u32), cudaMemcpyDeviceToHost));
+    raise_device_errors(flags);
+}
+
+void CUDASPHSimulator::raise_device_errors(u32 flags) {
     if (flags) {
         WCSPH_CUDA(cudaMemset(&st_.ptr->error_flags, 0, sizeof(u32)));
         if (flags & ERR_HASH_FULL) throw Error(WCSPH_ERR_HASH_FULL, "spatial hash table is full (raise table_size_mult)");
@@ -485,8 +489,11 @@ float CUDASPHSimulator::time_steps(int n, float delta) {
 }
 
 void CUDASPHSimulator::synchronize() {
+    // the flags come with the stream's work: one wait, no copy of its own after it
+    if (!flags_pinned_) WCSPH_CUDA(cudaMallocHost(&flags_pinned_, sizeof(u32)));
+    WCSPH_CUDA(cudaMemcpyAsync(flags_pinned_, &st_.ptr->error_flags, sizeof(u32), cudaMemcpyDeviceToHost, stream_));
     WCSPH_CUDA(cudaStreamSynchronize(stream_));
-    check_device_errors();
+    raise_device_errors(*flags_pinned_);
 }
 
 void CUDASPHSimulator::set_box(const wcsph_box& box) {

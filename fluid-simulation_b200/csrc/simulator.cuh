@@ -70,6 +70,10 @@ struct DevBuf {
         ptr = nullptr;
         count = 0;
     }
+    // alloc, keeping a buffer that has the size already (contents undefined)
+    void ensure(size_t n) {
+        if (count != n) alloc(n);
+    }
     size_t bytes() const { return count * sizeof(T); }
 };
 
@@ -194,6 +198,7 @@ private:
     void init_boundary(const float* bpos);
     void upload_state(const float* pos, const float* vel);
     void check_device_errors();
+    void raise_device_errors(u32 flags);
     void invalidate_graph();
     TravArgs trav_args(float delta);
     u32 fluid_table_size() const;
@@ -250,6 +255,7 @@ private:
     cudaEvent_t box_done_[kBoxSlots] = {};
     int box_slot_ = 0;
     float* metrics_pinned_ = nullptr;   // 2 floats: the metrics read-back
+    u32* flags_pinned_ = nullptr;       // the error flags' read-back
     DevBuf<float> metrics_dev_;
     // boundary
     DevBuf<float4> bpos_;
