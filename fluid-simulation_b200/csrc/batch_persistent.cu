@@ -93,7 +93,7 @@ size_t persistent_smem(const TravArgs& a) {
     const u32 ncell = static_cast<u32>((2 * a.range + 1) * (2 * a.range + 1) * (2 * a.range + 1));
     const bool wb = a.nb > 0;
     size_t b = sizeof(u32) * SORT_DIGITS * 256;                  // digit histograms
-    b = std::max(b, sizeof(u32) * (PWARPS * 256 + 256));          // onesweep ranks and bases
+    b = std::max(b, sizeof(sortdev::TileSmem));
     b = std::max(b, a.units ? sizeof(BlockSmem<PersistentBlock>) : PWARPS * warp_smem_bytes<PASS_DENSITY>(cap, ncell, wb));
     if (a.nbr == nullptr) {                                       // force and surface walk the bit matrix
         b = std::max(b, PWARPS * warp_smem_bytes<PASS_FORCE>(cap, ncell, wb));
@@ -140,10 +140,9 @@ __global__ void __launch_bounds__(PTHREADS, PERSISTENT_BLOCKS) persistent_ensemb
                 __syncthreads();
                 const u32 tile = s_tile;
                 if (tile >= ps.tiles) break;
-                sortdev::onesweep_tile(n, p, ps.keys[0], ps.keys[1], ps.keys[2], ps.vals[1], ps.vals[2], ps.offsets,
+                sortdev::onesweep_tile<u64, false>(n, p, ps.keys[0], ps.keys[1], ps.keys[2], ps.vals[1], ps.vals[2], ps.offsets,
                                        ps.lookback, ps.tiles, st, ps.spin_limit, 0u, tile,
-                                       reinterpret_cast<u32(*)[256]>(smem),
-                                       reinterpret_cast<u32*>(smem) + PWARPS * 256);
+                                            *reinterpret_cast<sortdev::TileSmem*>(smem));
                 __syncthreads();
             }
             if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;

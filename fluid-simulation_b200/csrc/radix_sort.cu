@@ -66,27 +66,24 @@ __global__ void keys_bounds_kernel(const float4* __restrict__ pos, u32 n, float 
     }
 }
 
-__global__ void compressed_keys_hist_kernel(const float4* __restrict__ pos, u32 n, float cs,
-                                            const DevState* __restrict__ st, u64* __restrict__ ckeys,
-                                            u32* __restrict__ hist) {
+__global__ void compressed_keys_hist_kernel(const u64* __restrict__ keys, u32 n, const DevState* __restrict__ st,
+                                            u64* __restrict__ ckeys, u32* __restrict__ hist) {
     __shared__ u32 s_hist[SORT_DIGITS][256];
     for (int t = threadIdx.x; t < SORT_DIGITS * 256; t += blockDim.x) (&s_hist[0][0])[t] = 0;
-    // smallest B with every cell coordinate in [-2^B, 2^B); B = 20 is the full key
-    const int lo = min(st->cell_lo[0], min(st->cell_lo[1], st->cell_lo[2]));
-    const int hi = max(st->cell_hi[0], max(st->cell_hi[1], st->cell_hi[2]));
-    int B = 0;
-    while (B < 20 && !(lo >= -(1 << B) && hi < (1 << B))) ++B;
+    const int B = sortdev::key_bits(st);
+    const bool narrow = sortdev::narrow_keys(st);
     const int ndigits = (3 * (B + 1) + 7) / 8;   // digits above are 0 for every key
+    const u64 low = (1ull << (3 * B)) - 1ull;    // bits 0..B-1 of every axis; the signs are bits 60..62
     u32 valid_keys = 0;
     __syncthreads();
     const u32 stride = gridDim.x * blockDim.x;
     // uniform trip count per warp (match.any); four loads in flight per thread
     for (u32 base = blockIdx.x * blockDim.x; base < n; base += 4 * stride) {
-        float4 x[4];
+        u64 full[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const u32 i = base + u * stride + threadIdx.x;
-            if (i < n) x[u] = pos[i];
+            if (i < n) full[u] = keys[i];
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -94,11 +91,9 @@ __global__ void compressed_keys_hist_kernel(const float4* __restrict__ pos, u32 
             const bool valid = i < n;
             u64 key = 0;
             if (valid) {
-                const int3 c = cell_of(x[u], cs);
-                key = part_by_3(static_cast<u32>(c.x + (1 << B))) |
-                      (part_by_3(static_cast<u32>(c.y + (1 << B))) << 1) |
-                      (part_by_3(static_cast<u32>(c.z + (1 << B))) << 2);
-                ckeys[i] = key;
+                key = (full[u] & low) | ((full[u] >> 60) << (3 * B));
+                if (narrow) reinterpret_cast<u32*>(ckeys)[i] = static_cast<u32>(key);
+                else ckeys[i] = key;
                 ++valid_keys;
             }
             sortdev::hist_add_key(s_hist, key, valid, ndigits);
@@ -139,17 +134,21 @@ __global__ void __launch_bounds__(SORT_THREADS)
 onesweep_kernel(u32 n, int pass, u64* __restrict__ k0, u64* __restrict__ k1, u64* __restrict__ k2,
                 u32* __restrict__ v1, u32* __restrict__ v2, const u32* __restrict__ offsets,
                 u32* __restrict__ lookback, u32 tiles, DevState* __restrict__ st, u32 spin_limit,
-                u32 stall_first_tile) {
+                u32 stall_first_tile, bool compressed) {
     if (!st->sort_active[pass]) return;
     __shared__ u32 s_tile;
-    __shared__ u32 s_wcnt[SORT_THREADS / 32][256];
-    __shared__ u32 s_base[256];
+    __shared__ sortdev::TileSmem S;
     if (threadIdx.x == 0) s_tile = atomicAdd(&st->sort_tile_counter[pass], 1u);
     __syncthreads();
     const u32 tile = s_tile;
     if (tile >= tiles) return;  // cannot happen: grid == tiles
-    sortdev::onesweep_tile(n, pass, k0, k1, k2, v1, v2, offsets, lookback, tiles, st, spin_limit,
-                           stall_first_tile, tile, s_wcnt, s_base);
+    if (compressed && st->sort_narrow)
+        sortdev::onesweep_tile<u32>(n, pass, reinterpret_cast<u32*>(k0), reinterpret_cast<u32*>(k1),
+                                    reinterpret_cast<u32*>(k2), v1, v2, offsets, lookback, tiles, st, spin_limit,
+                                    stall_first_tile, tile, S);
+    else
+        sortdev::onesweep_tile<u64>(n, pass, k0, k1, k2, v1, v2, offsets, lookback, tiles, st, spin_limit,
+                                    stall_first_tile, tile, S);
 }
 
 cudaError_t enqueue_sort_passes(const SortBuffers& b, u32 n, DevState* st, cudaStream_t stream) {
@@ -165,7 +164,7 @@ cudaError_t enqueue_sort_passes(const SortBuffers& b, u32 n, DevState* st, cudaS
     for (int p = 0; p < SORT_DIGITS; ++p) {
         onesweep_kernel<<<tiles, SORT_THREADS, 0, stream>>>(n, p, b.keys[0], b.keys[1], b.keys[2],
                                                             b.vals[1], b.vals[2], b.offsets, b.lookback,
-                                                            tiles, st, spin_limit, stall ? 1u : 0u);
+                                                            tiles, st, spin_limit, stall ? 1u : 0u, b.compressed);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

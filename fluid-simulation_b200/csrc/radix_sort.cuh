@@ -11,8 +11,13 @@
 //                 has a single non-empty bucket is constant over all keys and
 //                 its pass is skipped (the reference's 63-bit keys usually
 //                 vary in only 2-3 of the 8 digits); ping-pong buffer plan.
-//   onesweep    : per 2048-key tile: warp-level match.any ranking, per-digit
-//                 decoupled look-back across tiles (bounded spin), scatter.
+//   onesweep    : per 2048-key tile: warp-level match.any ranking, the tile
+//                 ordered by digit in shared memory, per-digit decoupled
+//                 look-back across tiles (bounded spin), write in runs.
+// Above 131,072 particles; smaller scenes take the cluster sort
+// (cluster_sort.cuh). Device time of a step's keys and sort: 1 M particles
+// 33 + 81 -> 27 + 71 us, 4 M 81 + 201 -> 64 + 150 (u32 words in runs; the
+// compression from the full keys instead of a second pass over the positions).
 // Buffers: keys[0] holds the input-order keys and is never overwritten (it is
 // the MORTON_KEYS parity field); passes alternate between keys[1]/keys[2]
 // and vals[1]/vals[2]. The first active pass generates the iota values.
@@ -40,6 +45,7 @@ struct SortBuffers {
     u32* offsets;     // [8][256] exclusive digit offsets
     u32* lookback;    // [8][tiles][256]
     u32 capacity;     // max keys
+    bool compressed;  // keys[0] comes from compressed_keys_hist_kernel (u32 words where they fit)
 };
 
 // Computes Morton keys of `pos` (cell = floorf(p / cs), particle_data.cuh:117-125)
@@ -52,7 +58,8 @@ __global__ void keys_hist_kernel(const float4* __restrict__ pos, u32 n, float cs
 //  * keys_bounds_kernel writes the reference's 63-bit Morton keys (the
 //    MORTON_KEYS field) and folds the cell-coordinate bounds into st;
 //  * compressed_keys_hist_kernel writes order-equivalent short keys for the
-//    sort and their digit histograms. With every cell coordinate c in
+//    sort (as u32 words where they fit) and their digit histograms, from the
+//    full keys alone: bits 0..B-1 of every axis and the signs. With every cell coordinate c in
 //    [-2^B, 2^B), the offset coordinate u = c + 2^20 has bits B..19 equal to
 //    NOT bit 20, so those bits never decide a Morton comparison; v = c + 2^B
 //    keeps exactly bits 0..B-1 and bit 20 (as bit B), and Morton(v) orders any
@@ -61,9 +68,8 @@ __global__ void keys_hist_kernel(const float4* __restrict__ pos, u32 n, float cs
 //    stable sort gives the same permutation.
 __global__ void keys_bounds_kernel(const float4* __restrict__ pos, u32 n, float cs, u64* __restrict__ keys_out,
                                    DevState* __restrict__ st);
-__global__ void compressed_keys_hist_kernel(const float4* __restrict__ pos, u32 n, float cs,
-                                            const DevState* __restrict__ st, u64* __restrict__ ckeys,
-                                            u32* __restrict__ hist);
+__global__ void compressed_keys_hist_kernel(const u64* __restrict__ keys, u32 n, const DevState* __restrict__ st,
+                                            u64* __restrict__ ckeys, u32* __restrict__ hist);
 // Histograms of already-computed keys (boundary sort, re-sorts).
 __global__ void hist_only_kernel(const u64* __restrict__ keys, u32 n, u32* __restrict__ hist);
 __global__ void sort_plan_kernel(u32 n, u32* __restrict__ hist, u32* __restrict__ offsets,
@@ -74,7 +80,8 @@ __global__ void sort_plan_kernel(u32 n, u32* __restrict__ hist, u32* __restrict_
 __global__ void onesweep_kernel(u32 n, int pass, u64* __restrict__ k0, u64* __restrict__ k1,
                                 u64* __restrict__ k2, u32* __restrict__ v1, u32* __restrict__ v2,
                                 const u32* __restrict__ offsets, u32* __restrict__ lookback,
-                                u32 tiles, DevState* __restrict__ st, u32 spin_limit, u32 stall_first_tile);
+                                u32 tiles, DevState* __restrict__ st, u32 spin_limit, u32 stall_first_tile,
+                                bool compressed);
 
 // Enqueues the complete sort (after keys[0] and hist are filled) on `stream`.
 // Returns the first enqueue error (cudaSuccess when every call was accepted).

@@ -369,6 +369,7 @@ void CUDASPHSimulator::enqueue_sort() {
     for (int i = 0; i < 3; ++i) { sb.keys[i] = keys_[i].ptr; sb.vals[i] = vals_[i].ptr; }
     sb.keys[0] = ckeys_.ptr;   // the sort reads the compressed keys; keys_[0] keeps the field
     sb.hist = hist_.ptr; sb.offsets = offsets_.ptr; sb.lookback = lookback_.ptr; sb.capacity = n_;
+    sb.compressed = true;
     WCSPH_CUDA(enqueue_sort_passes(sb, n_, st_.ptr, stream_));
 }
 
@@ -379,8 +380,7 @@ void CUDASPHSimulator::enqueue_keys() {
     // blocks more loads in flight (two per SM: 4 us more for the histograms)
     const u32 blocks = std::min<u32>((n + 255) / 256, 592);
     keys_bounds_kernel<<<blocks, 256, 0, stream_>>>(pos_a_.ptr, n, dp_.cell_size, keys_[0].ptr, st_.ptr);
-    compressed_keys_hist_kernel<<<blocks, 256, 0, stream_>>>(pos_a_.ptr, n, dp_.cell_size, st_.ptr, ckeys_.ptr,
-                                                             hist_.ptr);
+    compressed_keys_hist_kernel<<<blocks, 256, 0, stream_>>>(keys_[0].ptr, n, st_.ptr, ckeys_.ptr, hist_.ptr);
 }
 
 TravArgs CUDASPHSimulator::fixed_args(float dt) {

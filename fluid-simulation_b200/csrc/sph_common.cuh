@@ -174,15 +174,22 @@ __device__ __forceinline__ float4 external_force(float4 pos, const DevParams& P)
 
 // ------------------------------------------------------------ Morton keys --
 // part_by_3 / signed_to_unsigned / encode_morton (morton.cuh:7-34): 21 bits
-// per axis after a +2^20 offset, x | y<<1 | z<<2, 63-bit key.
-__host__ __device__ __forceinline__ u64 part_by_3(u64 n) {
-    n &= 0x1fffffull;
-    n = (n | (n << 32)) & 0x1f00000000ffffull;
-    n = (n | (n << 16)) & 0x1f0000ff0000ffull;
-    n = (n | (n << 8)) & 0x100f00f00f00f00full;
-    n = (n | (n << 4)) & 0x10c30c30c30c30c3ull;
-    n = (n | (n << 2)) & 0x1249249249249249ull;
-    return n;
+// per axis after a +2^20 offset, x | y<<1 | z<<2, 63-bit key. Bit b of an 11-bit
+// value goes to bit 3b; 21 bits are spread as 10 + 11, in 32-bit steps.
+__host__ __device__ __forceinline__ u32 spread11(u32 v) {
+    v &= 0x7ffu;
+    v = (v | (v << 16)) & 0x070000ffu;
+    v = (v | (v << 8)) & 0x0700f00fu;
+    v = (v | (v << 4)) & 0x430c30c3u;
+    v = (v | (v << 2)) & 0x49249249u;
+    return v;
+}
+// Bits 0..20 of x, y, z interleaved.
+__host__ __device__ __forceinline__ u64 interleave3(u32 x, u32 y, u32 z) {
+    const u32 lo = spread11(x & 0x3ffu) | (spread11(y & 0x3ffu) << 1) | (spread11(z & 0x3ffu) << 2);
+    const u64 hi = static_cast<u64>(spread11(x >> 10)) | (static_cast<u64>(spread11(y >> 10)) << 1) |
+                   (static_cast<u64>(spread11(z >> 10)) << 2);
+    return static_cast<u64>(lo) | (hi << 30);
 }
 __host__ __device__ __forceinline__ u32 offset_coord(int c) {
     return static_cast<u32>(c) + (1u << 20);
@@ -196,8 +203,7 @@ __device__ __forceinline__ int3 cell_of(float4 p, float cs) {
                      static_cast<int>(floorf(__fdiv_rn(p.z, cs))));
 }
 __host__ __device__ __forceinline__ u64 morton_key(int3 c) {
-    return part_by_3(offset_coord(c.x)) | (part_by_3(offset_coord(c.y)) << 1) |
-           (part_by_3(offset_coord(c.z)) << 2);
+    return interleave3(offset_coord(c.x), offset_coord(c.y), offset_coord(c.z));
 }
 
 // ------------------------------------------------------------- cell hash --
@@ -252,8 +258,8 @@ __host__ __device__ __forceinline__ u64 slot_hash(u64 pk) {
 // first differing bit of two keys sits at the same place in both. The stable
 // sort therefore gives every scene the permutation of its own single step.
 __host__ __device__ __forceinline__ u64 batch_key(u32 scene, int3 c) {
-    return (static_cast<u64>(scene) << 48) | part_by_3(static_cast<u32>(c.x + 32768)) |
-           (part_by_3(static_cast<u32>(c.y + 32768)) << 1) | (part_by_3(static_cast<u32>(c.z + 32768)) << 2);
+    return (static_cast<u64>(scene) << 48) | interleave3(static_cast<u32>(c.x + 32768), static_cast<u32>(c.y + 32768),
+                                                         static_cast<u32>(c.z + 32768));
 }
 constexpr int BATCH_CELL_LIMIT = 32768;   // batched cell coordinates lie in [-limit, limit)
 
@@ -309,6 +315,7 @@ struct DevState {
     u32 sort_sel[9];            // buffer read by pass p; sort_sel[8] = final
     u32 sort_tile_counter[8];
     u32 first_active;           // first active pass (generates the iota values)
+    u32 sort_narrow;            // the compressed keys are u32 words
     // density units (blocks of cells): listed by the reorder, claimed by the
     // density pass; both reset by the sort plan
     u32 unit_count;
