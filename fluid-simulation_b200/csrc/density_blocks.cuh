@@ -42,7 +42,9 @@ namespace {
 // 12 to 16 particles per cell (the 0.92-spaced, settled fluid holds 10.3);
 // denser blocks are split into smaller ones. The thread counts fit the rows of
 // a block into whole rounds: 4x4x4 cells hold 512 rows and a few (17 groups of
-// 32), two rounds of 9 warps and three of 8 (4 M particles: 853 us against 930).
+// 32), two rounds of 9 warps and three of 8 (4 M particles: 853 us against 930);
+// 4x4x2 cells one round of 9 and two of 8 (393 k with walls 125 -> 119, 12
+// scenes 0.285 -> 0.275 ms a step).
 template <int LEVEL>
 struct BlockCfg;
 template <>
@@ -51,7 +53,7 @@ struct BlockCfg<3> {   // 2x2x2 cells
 };
 template <>
 struct BlockCfg<5> {   // 4x4x2 cells
-    static constexpr int nt = 256, cap = 2048, words = 12, min_blocks = 4;
+    static constexpr int nt = 288, cap = 2048, words = 12, min_blocks = 3;
 };
 template <>
 struct BlockCfg<6> {   // 4x4x4 cells
@@ -221,7 +223,8 @@ __device__ __forceinline__ u32 density_staged_row(const DevParams& P, const Trav
             open = b < e0;
             if (!open) ++seg;
         }
-        // phase 2: the hits, in candidate order
+        // phase 2: the hits, in candidate order (two per turn, for independent
+        // chains, cost more than they hid: 1 M particles 204 -> 219 us)
         const bool listed = hits <= a.nbr_width;   // else the row's list is not used
         if (k) {
             u32 t = 0;

@@ -161,8 +161,8 @@ inline int list_warps(int kind, u32 n) { return n < LIST_SMALL ? 2 : (kind == 1 
 // and stage fewer cells per row (8, 4.5 and 3.4 candidates a row), smaller
 // ones give more thread blocks and a shorter last wave. Density pass in us at
 // levels 3 / 5 / 6: 33 k particles with walls 30 / 35 / 48, 79 k 53 / 65 / 80,
-// 393 k with walls 136 / 124 / 134, 0.7 M settled 246 / 260 / 251, 1 M
-// 254 / 226 / 208, 4 M 1092 / 1003 / 823.
+// 393 k with walls 136 / 119 / 128, 0.7 M settled 246 / 257 / 258, 1 M
+// 254 / 222 / 204, 4 M 1092 / 939 / 831.
 inline u32 unit_level(u32 n) { return n < (1u << 18) ? 3u : (n < (1u << 19) ? 5u : 6u); }
 
 void launch_pass(int kind, const DevParams& P, const TravArgs& a, cudaStream_t stream, int warps_per_block,
