@@ -6,7 +6,7 @@
 // Positions, velocities and particle ids are checkpointed every K steps.
 //
 // Backward, per segment (last first): the segment is re-run from its
-// checkpoint, each step with its own buffer set swapped in (sorted state,
+// checkpoint (the last one is still there from the forward), each step with its own buffer set swapped in (sorted state,
 // permutation, hash and cell ranges, neighbour bit matrix, density, pressure,
 // accelerations), so every step's neighbour sets are recomputed from the
 // checkpoint, not stored across the rollout. Then for each step in reverse,
@@ -164,6 +164,7 @@ struct Adjoint {
     int steps = 0, every = 0;
     float dt = 0.f;
     bool have_forward = false;
+    bool last_ready = false;         // seg holds the last segment's steps, as the forward ran them
     DevBuf<float4> ck_pos, ck_vel;   // [n_ckpt * n]
     DevBuf<u32> ck_ids;
     std::vector<StepSet> seg;        // one buffer set per step of a segment
@@ -177,9 +178,29 @@ struct Adjoint {
 
 void destroy_adjoint(void* adjoint) { delete static_cast<Adjoint*>(adjoint); }
 
+void adjoint_forget_steps(void* adjoint) {
+    if (adjoint) static_cast<Adjoint*>(adjoint)->last_ready = false;
+}
+
 static Adjoint& adj_of(void*& slot) {
     if (!slot) slot = new Adjoint();
     return *static_cast<Adjoint*>(slot);
+}
+
+// exchanges the context's step buffers with a segment step's set (pointer swaps)
+void CUDASPHSimulator::swap_step(StepSet& b) {
+    std::swap(pos_b_, b.pos_b); std::swap(vel_b_, b.vel_b); std::swap(ap_, b.ap); std::swap(vlap_, b.vlap);
+    std::swap(perm_, b.perm); std::swap(cstart_, b.cstart); std::swap(cend_, b.cend); std::swap(mask_, b.mask);
+    std::swap(ckey_, b.ckey); std::swap(table_, b.table); std::swap(rho_, b.rho); std::swap(prs_, b.prs);
+}
+
+// sizes a step's set as the context's buffers
+void CUDASPHSimulator::size_step(StepSet& b) {
+    const u32 n = n_;
+    b.pos_b.ensure(n); b.vel_b.ensure(n); b.ap.ensure(n); b.vlap.ensure(n);
+    b.perm.ensure(n); b.ckey.ensure(n); b.rho.ensure(n); b.prs.ensure(n);
+    b.table.ensure(table_size_); b.cstart.ensure(table_size_); b.cend.ensure(table_size_);
+    b.mask.ensure(mask_.count);
 }
 
 float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const float* target_host) {
@@ -196,12 +217,7 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
     A.ck_pos.ensure(static_cast<size_t>(nck) * n); A.ck_vel.ensure(static_cast<size_t>(nck) * n);
     A.ck_ids.ensure(static_cast<size_t>(nck) * n);
     if (static_cast<int>(A.seg.size()) != every) A.seg = std::vector<StepSet>(every);
-    for (StepSet& b : A.seg) {
-        b.pos_b.ensure(n); b.vel_b.ensure(n); b.ap.ensure(n); b.vlap.ensure(n);
-        b.perm.ensure(n); b.ckey.ensure(n); b.rho.ensure(n); b.prs.ensure(n);
-        b.table.ensure(table_size_); b.cstart.ensure(table_size_); b.cend.ensure(table_size_);
-        b.mask.ensure(mask_.count);
-    }
+    for (StepSet& b : A.seg) size_step(b);
     A.ids_a.ensure(n); A.ids_b.ensure(n);
     A.target.ensure(n); A.final_pos.ensure(n); A.final_vel.ensure(n);
     A.xbar.ensure(n); A.vbar.ensure(n); A.xbar_s.ensure(n); A.vbar_s.ensure(n); A.abar.ensure(n); A.w.ensure(n);
@@ -219,11 +235,29 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
                                    cudaMemcpyDeviceToDevice, stream_));
     };
     ckpt(0);
+    A.have_forward = false;
+    A.last_ready = false;
+    const int last0 = steps > 0 ? (steps - 1) / every * every : 0;   // first step of the last segment
     for (int s = 0; s < steps; ++s) {
+        // the steps of the last segment run in their own buffer sets, where the
+        // backward pass expects them; the very last one in the context's (whose
+        // fields the caller may read) and is copied
+        const bool own_set = s >= last0 && s + 1 < steps;
+        if (own_set) swap_step(A.seg[s - last0]);
         enqueue_fixed_step(dt);
         ids_gather_kernel<<<blocks(n), 256, 0, stream_>>>(A.ids_a.ptr, perm_.ptr, A.ids_b.ptr, n);
+        if (own_set) swap_step(A.seg[s - last0]);
         std::swap(A.ids_a, A.ids_b);
         if ((s + 1) % every == 0) ckpt((s + 1) / every);
+    }
+    if (steps > 0) {
+        StepSet& b = A.seg[steps - 1 - last0];
+        auto keep = [this](auto& to, const auto& from) {
+            WCSPH_CUDA(cudaMemcpyAsync(to.ptr, from.ptr, from.bytes(), cudaMemcpyDeviceToDevice, stream_));
+        };
+        keep(b.pos_b, pos_b_); keep(b.vel_b, vel_b_); keep(b.ap, ap_); keep(b.vlap, vlap_);
+        keep(b.perm, perm_); keep(b.cstart, cstart_); keep(b.cend, cend_); keep(b.mask, mask_);
+        keep(b.ckey, ckey_); keep(b.table, table_); keep(b.rho, rho_); keep(b.prs, prs_);
     }
     WCSPH_CUDA(cudaMemcpyAsync(A.final_pos.ptr, pos_a_.ptr, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream_));
     WCSPH_CUDA(cudaMemcpyAsync(A.final_vel.ptr, vel_a_.ptr, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream_));
@@ -234,6 +268,7 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
     WCSPH_CUDA(cudaMemcpyAsync(&loss, A.accum.ptr, sizeof(double), cudaMemcpyDeviceToHost, stream_));
     synchronize();
     A.have_forward = true;
+    A.last_ready = steps > 0;
     stepped_since_state_ = true;
     return static_cast<float>(loss / static_cast<double>(n));
 }
@@ -244,12 +279,7 @@ void CUDASPHSimulator::rollout_backward(float* grad_v0, float* grad_visc, float*
     Adjoint& A = *static_cast<Adjoint*>(adjoint_);
     const u32 n = n_;
     const float dt = A.dt;
-    // exchanges the context's step buffers with a segment step's set (pointer swaps)
-    auto swap_step = [this](StepSet& b) {
-        std::swap(pos_b_, b.pos_b); std::swap(vel_b_, b.vel_b); std::swap(ap_, b.ap); std::swap(vlap_, b.vlap);
-        std::swap(perm_, b.perm); std::swap(cstart_, b.cstart); std::swap(cend_, b.cend); std::swap(mask_, b.mask);
-        std::swap(ckey_, b.ckey); std::swap(table_, b.table); std::swap(rho_, b.rho); std::swap(prs_, b.prs);
-    };
+    for (StepSet& b : A.seg) size_step(b);   // the configuration may have changed since the forward
     const float np_dt = dt < params_.non_pressure_max_time_step ? dt : params_.non_pressure_max_time_step;
     // dL/dx_T in the final state order, dL/dv_T = 0
     WCSPH_CUDA(cudaMemsetAsync(A.accum.ptr, 0, sizeof(double) * 3, stream_));
@@ -264,7 +294,8 @@ void CUDASPHSimulator::rollout_backward(float* grad_v0, float* grad_visc, float*
                                    cudaMemcpyDeviceToDevice, stream_));
         WCSPH_CUDA(cudaMemcpyAsync(vel_a_.ptr, A.ck_vel.ptr + static_cast<size_t>(seg) * n, sizeof(float4) * n,
                                    cudaMemcpyDeviceToDevice, stream_));
-        for (int s = s0; s < s1; ++s) {  // re-run the segment, each step into its own buffer set
+        const bool ready = A.last_ready && seg == nseg - 1;   // the forward left this segment's steps
+        for (int s = s0; s < s1 && !ready; ++s) {  // re-run the segment, each step into its own buffer set
             swap_step(A.seg[s - s0]);
             enqueue_fixed_step(dt);
             swap_step(A.seg[s - s0]);
@@ -290,6 +321,7 @@ void CUDASPHSimulator::rollout_backward(float* grad_v0, float* grad_visc, float*
             swap_step(A.seg[s - s0]);
         }
     }
+    A.last_ready = A.last_ready && nseg == 1;   // earlier segments were run into the same sets
     double acc[3];
     WCSPH_CUDA(cudaMemcpyAsync(acc, A.accum.ptr, sizeof(double) * 3, cudaMemcpyDeviceToHost, stream_));
     if (grad_v0)

@@ -128,6 +128,10 @@ public:
 
 class Tuner;  // tuner.cuh
 void destroy_adjoint(void* adjoint);  // adjoint.cu
+// The steps a rollout's forward left for its backward no longer apply (box,
+// parameters or configuration changed): the backward re-runs them.
+void adjoint_forget_steps(void* adjoint);
+struct StepSet;   // adjoint.cu
 
 class CUDASPHSimulator final : public FluidSimulator {
 public:
@@ -199,6 +203,8 @@ private:
     void upload_state(const float* pos, const float* vel);
     void check_device_errors();
     void raise_device_errors(u32 flags);
+    void swap_step(StepSet& b);
+    void size_step(StepSet& b);
     void invalidate_graph();
     TravArgs trav_args(float delta);
     u32 fluid_table_size() const;
