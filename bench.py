@@ -338,12 +338,13 @@ def bench_batched(args, n_scenes: int = 256, steps: int = 500):
         sim.step_n(steps, 1e-3)
         sim.synchronize()
     seq_s = time.perf_counter() - t0
+    seq_launches = sum(sim.launches_per_step() for sim in sims) * steps
     for sim in sims:
         sim.close()
     out["value"] = out["persistent"]
     out["sequential_value"] = total * steps / seq_s
     out["gain"] = out["value"] / out["sequential_value"]
-    out["launches"] = {"persistent": 1, "per_stage": 14 * steps, "sequential": 14 * n_scenes * steps}
+    out["launches"] = {"persistent": 1, "per_stage": 14 * steps, "sequential": seq_launches}
     return out
 
 
