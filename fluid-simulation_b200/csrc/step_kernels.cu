@@ -52,7 +52,7 @@ density_block_kernel(const DevParams P, const TravArgs a) {
 // Neighbours summed together (list_rows' DEPTH) and resident warps per SM the
 // register allocation of the list kernels must allow (36 -> 56 registers, 48 ->
 // 40). Both passes wait on neighbour gathers.
-// Above 2^18 particles the force pass sums two neighbours at a time, with the
+// From 2^17 particles on the force pass sums two neighbours at a time, with the
 // next two in flight, and gains more than the warps it costs: 1 M particles
 // 141 -> 121 us, 4 M 497 -> 430 (28 warps 126 / 461, 40 warps spill: 166 / 629,
 // three at a time 136 / 505). The surface pass keeps one at a time, all the

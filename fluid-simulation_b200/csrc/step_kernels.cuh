@@ -154,7 +154,10 @@ void launch_reorder_cells(const float4* pos_in, const float4* vel_in, const u32*
 // Below this many particles the list passes run their few-warps-per-SM variant
 // (ListCfg), best in 2-warp blocks; above, the force pass takes 4-warp blocks
 // and the surface pass 8-warp blocks.
-constexpr u32 LIST_SMALL = 1u << 18;
+// Force / surface in us, few-warps variant against the other: 79 k 27 / 25
+// against 55 / 55 before it, 135 k 34 / 34 against 30 / 28, 198 k 40 / 50
+// against 42 / 40, 250 k 44-48 / 50-56 against 44-46 / 52-58.
+constexpr u32 LIST_SMALL = 1u << 17;
 inline int list_warps(int kind, u32 n) { return n < LIST_SMALL ? 2 : (kind == 1 ? 4 : 8); }
 
 // Cells per density unit (BlockCfg), as a power of two. Larger units look up
