@@ -113,12 +113,21 @@ class ClockSampler:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.device}", f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits",
-                 "-lms", "200"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+                 "-lms", "20"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
         except Exception:
             self.proc = None
         return self
+
+    def wait_first(self, busy, limit_s: float = 3.0):
+        """Runs `busy` (keeps the clocks up) until the sampler delivers, then
+        drops those samples: the timed region starts with the sampler running
+        (a step takes well under a millisecond, the sampler's start a hundred)."""
+        t0 = time.perf_counter()
+        while self.proc is not None and not self.rows and time.perf_counter() - t0 < limit_s:
+            busy()
+        self.rows.clear()
 
     def _read(self):
         for line in self.proc.stdout:
@@ -228,7 +237,16 @@ def run_ours(args, world, rank, local, dist):
     torch.cuda.synchronize(local)
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
+    scratch = torch.zeros(1 << 26, device=f"cuda:{local}")
+
+    def busy():
+        scratch.add_(1.0)
+        torch.cuda.synchronize(local)
+
     with ClockSampler(local) as clk:
+        clk.wait_first(busy)
+        barrier(dist, local)
+        torch.cuda.synchronize(local)
         e0.record(stream)
         for k in range(args.warmup, args.warmup + args.steps):
             one(k)
