@@ -39,7 +39,7 @@ __global__ void ids_gather_kernel(const u32* __restrict__ ids_in, const u32* __r
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const u32 j = perm[i];
-        if (j < n) ids_out[i] = ids_in[j];   // always true unless the step's sort failed (reported)
+        ids_out[i] = ids_in[j < n ? j : i];   // always j unless the step's sort failed (reported)
     }
 }
 
@@ -194,13 +194,20 @@ void CUDASPHSimulator::swap_step(StepSet& b) {
     std::swap(ckey_, b.ckey); std::swap(table_, b.table); std::swap(rho_, b.rho); std::swap(prs_, b.prs);
 }
 
-// sizes a step's set as the context's buffers
+// sizes a step's set as the context's buffers. New buffers start as the
+// context's do (valid indices, an empty hash): a step whose sort fails leaves
+// them as they were, and nothing may then read an index past n.
 void CUDASPHSimulator::size_step(StepSet& b) {
+    auto size = [this](auto& buf, size_t count, int fill) {
+        if (buf.count == count) return;
+        buf.alloc(count);
+        if (count) WCSPH_CUDA(cudaMemsetAsync(buf.ptr, fill, buf.bytes(), stream_));
+    };
     const u32 n = n_;
-    b.pos_b.ensure(n); b.vel_b.ensure(n); b.ap.ensure(n); b.vlap.ensure(n);
-    b.perm.ensure(n); b.ckey.ensure(n); b.rho.ensure(n); b.prs.ensure(n);
-    b.table.ensure(table_size_); b.cstart.ensure(table_size_); b.cend.ensure(table_size_);
-    b.mask.ensure(mask_.count);
+    size(b.pos_b, n, 0); size(b.vel_b, n, 0); size(b.ap, n, 0); size(b.vlap, n, 0);
+    size(b.perm, n, 0); size(b.ckey, n, 0); size(b.rho, n, 0); size(b.prs, n, 0);
+    size(b.table, table_size_, 0xff); size(b.cstart, table_size_, 0); size(b.cend, table_size_, 0);
+    size(b.mask, mask_.count, 0);
 }
 
 float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const float* target_host) {

@@ -1,0 +1,39 @@
+"""Error paths of the differentiable rollout: a step whose sort fails, and a
+forward pass that fails before it has run. Nothing here faults or hangs."""
+import numpy as np
+import pytest
+
+import wcsph
+from test_gpu_adjoint import rollout_scene
+
+pytestmark = pytest.mark.gpu
+
+
+def rollout(sim, target, steps=6, every=3):
+    loss = sim.rollout_forward(steps, 1e-3, every, target)
+    return loss, sim.rollout_backward()[0]
+
+
+# the failed steps run in the context's buffers, in their own sets, or both; on
+# a context that has no rollout's workspaces yet, and on one that has
+@pytest.mark.parametrize("every", [1, 3, 6])
+@pytest.mark.parametrize("used", [False, True])
+def test_sort_timeout_in_a_rollout(every, used):
+    p, bx, pos, walls, target = rollout_scene(dims=(16, 16, 24))   # 6,144 particles: 3 sort tiles
+    with wcsph.CUDASPHSimulator(p, pos, bx, boundary_pos=walls) as sim:
+        want = rollout(sim, target)
+    with wcsph.CUDASPHSimulator(p, pos, bx, boundary_pos=walls) as sim:
+        if used:
+            rollout(sim, target, 2, every)
+            sim.set_state(pos)
+        with wcsph.stall_sort():
+            with pytest.raises(wcsph.WcsphError) as e:
+                sim.rollout_forward(6, 1e-3, every, target)
+        assert e.value.status == wcsph.ERR_DEVICE_TIMEOUT
+        with pytest.raises(wcsph.WcsphError) as e:
+            sim.rollout_backward()
+        assert e.value.status == wcsph.ERR_STATE
+        x, v = sim.get_state()
+        assert np.array_equal(x, pos) and not v.any()   # the failed steps left the state as it was
+        got = rollout(sim, target)                      # and the context works on
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
