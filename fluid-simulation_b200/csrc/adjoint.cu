@@ -196,10 +196,13 @@ void CUDASPHSimulator::swap_step(StepSet& b) {
 
 // sizes a step's set as the context's buffers. New buffers start as the
 // context's do (valid indices, an empty hash): a step whose sort fails leaves
-// them as they were, and nothing may then read an index past n.
-void CUDASPHSimulator::size_step(StepSet& b) {
-    auto size = [this](auto& buf, size_t count, int fill) {
+// them as they were, and nothing may then read an index past n. Returns whether
+// the set is as it was (no buffer is new).
+bool CUDASPHSimulator::size_step(StepSet& b) {
+    bool same = true;
+    auto size = [&](auto& buf, size_t count, int fill) {
         if (buf.count == count) return;
+        same = false;
         buf.alloc(count);
         if (count) WCSPH_CUDA(cudaMemsetAsync(buf.ptr, fill, buf.bytes(), stream_));
     };
@@ -208,6 +211,7 @@ void CUDASPHSimulator::size_step(StepSet& b) {
     size(b.perm, n, 0); size(b.ckey, n, 0); size(b.rho, n, 0); size(b.prs, n, 0);
     size(b.table, table_size_, 0xff); size(b.cstart, table_size_, 0); size(b.cend, table_size_, 0);
     size(b.mask, mask_.count, 0);
+    return same;
 }
 
 float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const float* target_host) {
@@ -216,6 +220,10 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
     if (params_.external_force != WCSPH_FORCE_NONE && params_.external_force != WCSPH_FORCE_CONSTANT)
         throw Error(WCSPH_ERR_NOT_SUPPORTED, "the differentiable rollout supports no or constant external force");
     Adjoint& A = adj_of(adjoint_);
+    // no rollout to go back through until this one has run: the counts and the
+    // workspaces change below, and an allocation may fail half way
+    A.have_forward = false;
+    A.last_ready = false;
     const u32 n = n_;
     const int nck = steps / every + 1;
     A.steps = steps; A.every = every; A.dt = dt;
@@ -242,8 +250,6 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
                                    cudaMemcpyDeviceToDevice, stream_));
     };
     ckpt(0);
-    A.have_forward = false;
-    A.last_ready = false;
     const int last0 = steps > 0 ? (steps - 1) / every * every : 0;   // first step of the last segment
     for (int s = 0; s < steps; ++s) {
         // the steps of the last segment run in their own buffer sets, where the
@@ -286,7 +292,8 @@ void CUDASPHSimulator::rollout_backward(float* grad_v0, float* grad_visc, float*
     Adjoint& A = *static_cast<Adjoint*>(adjoint_);
     const u32 n = n_;
     const float dt = A.dt;
-    for (StepSet& b : A.seg) size_step(b);   // the configuration may have changed since the forward
+    for (StepSet& b : A.seg)   // the configuration may have changed since the forward
+        if (!size_step(b)) A.last_ready = false;
     const float np_dt = dt < params_.non_pressure_max_time_step ? dt : params_.non_pressure_max_time_step;
     // dL/dx_T in the final state order, dL/dv_T = 0
     WCSPH_CUDA(cudaMemsetAsync(A.accum.ptr, 0, sizeof(double) * 3, stream_));

@@ -59,6 +59,7 @@ struct DevBuf {
         if (n == 0) return;
         const cudaError_t e = cudaMalloc(&ptr, n * sizeof(T));
         if (e != cudaSuccess) {
+            cudaGetLastError();   // reported here; a later launch check must not see it
             ptr = nullptr;
             throw Error(e == cudaErrorMemoryAllocation ? WCSPH_ERR_OUT_OF_MEMORY : WCSPH_ERR_CUDA,
                         std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
@@ -204,7 +205,7 @@ private:
     void check_device_errors();
     void raise_device_errors(u32 flags);
     void swap_step(StepSet& b);
-    void size_step(StepSet& b);
+    bool size_step(StepSet& b);
     void invalidate_graph();
     TravArgs trav_args(float delta);
     u32 fluid_table_size() const;

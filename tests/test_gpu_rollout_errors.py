@@ -37,3 +37,22 @@ def test_sort_timeout_in_a_rollout(every, used):
         assert np.array_equal(x, pos) and not v.any()   # the failed steps left the state as it was
         got = rollout(sim, target)                      # and the context works on
     assert got[0] == want[0] and np.array_equal(got[1], want[1])
+
+
+# the second forward fails before it has run (its checkpoints would take 8 TB:
+# the allocation is refused at once); the rollout before it is no longer there
+def test_forward_out_of_memory_leaves_no_rollout_behind():
+    p, bx, pos, walls, target = rollout_scene(dims=(8, 8, 8))
+    with wcsph.CUDASPHSimulator(p, pos, bx, boundary_pos=walls) as sim:
+        want = rollout(sim, target)
+        sim.set_state(pos)
+        with pytest.raises(wcsph.WcsphError) as e:
+            sim.rollout_forward(1 << 30, 1e-3, 1, target)
+        assert e.value.status == wcsph.ERR_OUT_OF_MEMORY
+        with pytest.raises(wcsph.WcsphError) as e:
+            sim.rollout_backward()
+        assert e.value.status == wcsph.ERR_STATE
+        x, v = sim.get_state()
+        assert np.array_equal(x, pos) and not v.any()
+        got = rollout(sim, target)
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
