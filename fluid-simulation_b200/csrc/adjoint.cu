@@ -6,10 +6,12 @@
 // Positions, velocities and particle ids are checkpointed every K steps.
 //
 // Backward, per segment (last first): the segment is re-run from its
-// checkpoint (the last one is still there from the forward), each step with its own buffer set swapped in (sorted state,
-// permutation, hash and cell ranges, neighbour bit matrix, density, pressure,
-// accelerations), so every step's neighbour sets are recomputed from the
-// checkpoint, not stored across the rollout. Then for each step in reverse,
+// checkpoint (the last one is still there from the forward), under the
+// parameters, box and configuration of the forward, each step with its own
+// buffer set swapped in (sorted state, permutation, hash and cell ranges,
+// neighbour bit matrix, density, pressure, accelerations), so every step's
+// neighbour sets are recomputed from the checkpoint, not stored across the
+// rollout. Then for each step in reverse,
 // with that step's set swapped in again, the adjoint kernels run:
 //   adj_integrate   reverse of box collision and symplectic Euler (per particle)
 //   ADJ_FORCE pass  reverse of the symmetric pressure force (+boundary term),
@@ -165,6 +167,9 @@ struct Adjoint {
     float dt = 0.f;
     bool have_forward = false;
     bool last_ready = false;         // seg holds the last segment's steps, as the forward ran them
+    wcsph_params params{};           // what the forward ran with: the backward re-runs its steps
+    DevBox box{};                    // under the same, whatever has been set since
+    StepConfig cfg{};
     DevBuf<float4> ck_pos, ck_vel;   // [n_ckpt * n]
     DevBuf<u32> ck_ids;
     std::vector<StepSet> seg;        // one buffer set per step of a segment
@@ -177,10 +182,6 @@ struct Adjoint {
 };
 
 void destroy_adjoint(void* adjoint) { delete static_cast<Adjoint*>(adjoint); }
-
-void adjoint_forget_steps(void* adjoint) {
-    if (adjoint) static_cast<Adjoint*>(adjoint)->last_ready = false;
-}
 
 static Adjoint& adj_of(void*& slot) {
     if (!slot) slot = new Adjoint();
@@ -227,6 +228,7 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
     const u32 n = n_;
     const int nck = steps / every + 1;
     A.steps = steps; A.every = every; A.dt = dt;
+    A.params = params_; A.box = box_host_; A.cfg = cfg_;
     // workspaces are kept from one rollout to the next (an optimisation calls this
     // once per iteration with the same sizes)
     A.ck_pos.ensure(static_cast<size_t>(nck) * n); A.ck_vel.ensure(static_cast<size_t>(nck) * n);
@@ -286,14 +288,39 @@ float CUDASPHSimulator::rollout_forward(int steps, float dt, int every, const fl
     return static_cast<float>(loss / static_cast<double>(n));
 }
 
+// Parameters, box and configuration as a rollout's forward had them. The order
+// that a step sorts into depends on them (cell size, trajectory), and the
+// gradients are carried back row by row, so a re-run under others would hand
+// them to other particles.
+void CUDASPHSimulator::set_setup(const wcsph_params& p, const DevBox& box, const StepConfig& c) {
+    if (std::memcmp(&p, &params_, sizeof p) != 0) set_params(p);
+    apply_config(c);   // nothing to do for the same one
+    if (std::memcmp(&box, &box_host_, sizeof box) != 0) upload_box(box);
+}
+
 void CUDASPHSimulator::rollout_backward(float* grad_v0, float* grad_visc, float* grad_stiff) {
     if (!adjoint_ || !static_cast<Adjoint*>(adjoint_)->have_forward)
         throw Error(WCSPH_ERR_STATE, "rollout_backward needs a rollout_forward first");
+    const Adjoint& A = *static_cast<Adjoint*>(adjoint_);
+    const wcsph_params params = params_;
+    const DevBox box = box_host_;
+    const StepConfig cfg = cfg_;
+    try {
+        set_setup(A.params, A.box, A.cfg);
+        run_backward(grad_v0, grad_visc, grad_stiff);
+    } catch (...) {
+        set_setup(params, box, cfg);
+        throw;
+    }
+    set_setup(params, box, cfg);
+}
+
+void CUDASPHSimulator::run_backward(float* grad_v0, float* grad_visc, float* grad_stiff) {
     Adjoint& A = *static_cast<Adjoint*>(adjoint_);
     const u32 n = n_;
     const float dt = A.dt;
-    for (StepSet& b : A.seg)   // the configuration may have changed since the forward
-        if (!size_step(b)) A.last_ready = false;
+    for (StepSet& b : A.seg)
+        if (!size_step(b)) A.last_ready = false;   // the sets hold other steps, or none
     const float np_dt = dt < params_.non_pressure_max_time_step ? dt : params_.non_pressure_max_time_step;
     // dL/dx_T in the final state order, dL/dv_T = 0
     WCSPH_CUDA(cudaMemsetAsync(A.accum.ptr, 0, sizeof(double) * 3, stream_));

@@ -497,8 +497,11 @@ void CUDASPHSimulator::synchronize() {
 }
 
 void CUDASPHSimulator::set_box(const wcsph_box& box) {
-    adjoint_forget_steps(adjoint_);
-    box_host_ = make_dev_box(box);
+    upload_box(make_dev_box(box));
+}
+
+void CUDASPHSimulator::upload_box(const DevBox& box) {
+    box_host_ = box;
     if (!box_pinned_) {
         WCSPH_CUDA(cudaMallocHost(&box_pinned_, sizeof(DevBox) * kBoxSlots));
         for (cudaEvent_t& e : box_done_) WCSPH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -513,7 +516,6 @@ void CUDASPHSimulator::set_box(const wcsph_box& box) {
 
 void CUDASPHSimulator::set_params(const wcsph_params& p) {
     validate_params(p);
-    adjoint_forget_steps(adjoint_);
     if (p.particle_radius != params_.particle_radius)
         throw Error(WCSPH_ERR_INVALID_ARGUMENT, "particle_radius cannot change after creation");
     params_ = p;
@@ -542,7 +544,6 @@ void CUDASPHSimulator::apply_config(const StepConfig& c) {
         throw Error(WCSPH_ERR_CONFIG, "particles_per_warp must be 8, 16 or 32");
     if (c.nbr_width < 0 || c.nbr_width > 1024)
         throw Error(WCSPH_ERR_CONFIG, "neighbour_list_width must be in [0, 1024]");
-    adjoint_forget_steps(adjoint_);
     cfg_ = c;
     params_.cell_size_mult = c.cell_size_mult;
     params_.table_size_mult = c.table_size_mult;

@@ -129,9 +129,6 @@ public:
 
 class Tuner;  // tuner.cuh
 void destroy_adjoint(void* adjoint);  // adjoint.cu
-// The steps a rollout's forward left for its backward no longer apply (box,
-// parameters or configuration changed): the backward re-runs them.
-void adjoint_forget_steps(void* adjoint);
 struct StepSet;   // adjoint.cu
 
 class CUDASPHSimulator final : public FluidSimulator {
@@ -206,6 +203,9 @@ private:
     void raise_device_errors(u32 flags);
     void swap_step(StepSet& b);
     bool size_step(StepSet& b);
+    void set_setup(const wcsph_params& p, const DevBox& box, const StepConfig& c);
+    void run_backward(float* grad_v0, float* grad_visc, float* grad_stiff);
+    void upload_box(const DevBox& box);
     void invalidate_graph();
     TravArgs trav_args(float delta);
     u32 fluid_table_size() const;

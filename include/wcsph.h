@@ -335,7 +335,8 @@ const char* wcsph_batch_last_error(const wcsph_batch* b);
  * Fixed dt (CFL off), surface tension must be 0. Forward stores positions and
  * velocities every `checkpoint_every` steps; backward recomputes each segment
  * (sort + neighbourhood search again from the checkpoint) and runs the
- * hand-written adjoint kernels in reverse.
+ * hand-written adjoint kernels in reverse, under the parameters, box and
+ * configuration of the forward (what was set since applies again afterwards).
  * Loss = mean_i |x_T,i - target_i|^2 (targets indexed by initial particle id).
  * Outputs: dL/dv0 (float4 per initial particle id), dL/dnu, dL/dk.          */
 int wcsph_rollout_forward(wcsph_ctx* ctx, int steps, float dt, int checkpoint_every,

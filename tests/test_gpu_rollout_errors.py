@@ -56,3 +56,50 @@ def test_forward_out_of_memory_leaves_no_rollout_behind():
         assert np.array_equal(x, pos) and not v.any()
         got = rollout(sim, target)
     assert got[0] == want[0] and np.array_equal(got[1], want[1])
+
+
+def other_parameters(sim, p, bx):
+    q = wcsph.Params.from_buffer_copy(p)
+    q.cell_size_mult, q.table_size_mult = 0.5, 8    # another sort order, another table
+    q.viscosity *= 3
+    q.rest_density *= 1.1                           # other boundary masses
+    sim.set_params(q)
+
+
+def other_box(sim, p, bx):
+    sim.set_box(wcsph.box((0, 0, 0), (0.25, 0.2, 0.15), wcsph.rotation_z(0.2)))
+
+
+# what is set between forward and backward changes neither the gradients nor,
+# afterwards, what was set: the next step is that of a context that had no backward
+@pytest.mark.parametrize("every", [2, 5])
+@pytest.mark.parametrize("between", [other_parameters, other_box, lambda sim, p, bx: sim.update(1e-3)])
+def test_backward_is_the_forwards(every, between):
+    p, bx, pos, walls, target = rollout_scene(dims=(10, 9, 8))
+
+    def run(change, backward):
+        with wcsph.CUDASPHSimulator(p, pos, bx, boundary_pos=walls) as sim:
+            sim.rollout_forward(5, 1e-3, every, target)
+            if change:
+                between(sim, p, bx)
+            grads = sim.rollout_backward() if backward else None
+            if change and backward:   # from the rollout's end, under what was set
+                sim.rollout_forward(2, 1e-3, 1, target)
+            return grads, sim.get_state()
+
+    def forward_again():
+        with wcsph.CUDASPHSimulator(p, pos, bx, boundary_pos=walls) as sim:
+            sim.rollout_forward(5, 1e-3, every, target)
+            x, v = sim.get_state()
+            between(sim, p, bx)
+            sim.set_state(x, v)
+            sim.rollout_forward(2, 1e-3, 1, target)
+            return sim.get_state()
+
+    (gv0, gnu0, gk0), _ = run(False, True)
+    (gv, gnu, gk), after = run(True, True)
+    assert np.array_equal(gv, gv0)
+    # the two scalars are double sums in arrival order, rounded to float
+    assert abs(gnu - gnu0) <= 2e-7 * abs(gnu0) and abs(gk - gk0) <= 2e-7 * abs(gk0)
+    want = forward_again()
+    assert np.array_equal(after[0], want[0]) and np.array_equal(after[1], want[1])
