@@ -114,25 +114,38 @@ __device__ __forceinline__ void density_boundary_row(const DevParams& P, const T
     if (a.bmask != nullptr) a.bmask[i] = make_uint4(mk[0], mk[1], mk[2], mk[3]);
 }
 
-// Sum of W of one pair: 2 (1 - q)^3 - max(1 - 2 q, 0)^3 is the cubic spline
-// over its factor for q <= 1; the two cubes are summed apart. The rounding is
-// written out: every kernel that inlines this produces the same bits.
-__device__ __forceinline__ void density_pair(float r2, const DevParams& P, float& t3, float& u3) {
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(r2));
-    const float q = __fmul_rn(r, P.inv_h);
-    const float t = __fsub_rn(1.f, q);
-    const float u = fmaxf(__fmaf_rn(-2.f, q, 1.f), 0.f);
-    t3 = __fmaf_rn(__fmul_rn(t, t), t, t3);
-    u3 = __fmaf_rn(__fmul_rn(u, u), u, u3);
-}
+// Sum of W over a row's pairs: 2 (1 - q)^3 - max(1 - 2 q, 0)^3 is the cubic
+// spline over its factor for q <= 1; the two cubes are summed apart. The first
+// sum is a single chain of 25 to 100 terms, so its rounding errors are carried
+// along (Kahan); few pairs are within h / 2, so the second is short. RMS error of
+// rho against 64 bits, of the lane-run sums this pass had before / plain chains
+// with q from sqrt.approx / as it is: 0.7 M settled 7.8e-5 / 9.4e-5 / 6.3e-5,
+// 1 M lattice 5.4e-5 / 6.3e-5 / 4.6e-5, 79 k 2.09e-4 / 2.33e-4 / 2.05e-4; it costs
+// 1 M settled 737 -> 753 us a step and the persistent ensemble 3 %. The rounding
+// is written out: every kernel that inlines this produces the same bits.
+struct DensitySum {
+    float t3 = 0.f, over = 0.f;   // sum of (1 - q)^3, and by how much it is over
+    float u3 = 0.f;
+    __device__ __forceinline__ void pair(float r2, const DevParams& P) {
+        float rinv;
+        const float q = q_of(r2, rinv, P);
+        const float t = __fsub_rn(1.f, q);
+        const float u = fmaxf(__fmaf_rn(-2.f, q, 1.f), 0.f);
+        const float term = __fmaf_rn(__fmul_rn(t, t), t, -over);
+        const float sum = __fadd_rn(t3, term);
+        over = __fsub_rn(__fsub_rn(sum, t3), term);
+        t3 = sum;
+        u3 = __fmaf_rn(__fmul_rn(u, u), u, u3);
+    }
+    __device__ __forceinline__ float value() const { return __fmaf_rn(2.f, t3, -__fmaf_rn(2.f, over, u3)); }
+};
 
 // Row i without staged candidates (a single cell whose 27 cells exceed the
 // capacity): its cells one after the other from global memory, in the same
 // order. Returns the neighbour count.
 template <bool BATCH>
 __device__ __forceinline__ u32 density_direct_row(const DevParams& P, const TravArgs& a, u32 i, u64 pk, float4 xi,
-                                                  float& t3, float& u3) {
+                                                  DensitySum& W) {
     u32 ux, uy, uz, scene;
     decode_cell<BATCH>(pk, ux, uy, uz, scene);
     u32 hits = 0;
@@ -150,7 +163,7 @@ __device__ __forceinline__ u32 density_direct_row(const DevParams& P, const Trav
             if (!(r2 <= P.h2) || j == i) continue;
             if (hits < a.nbr_width) a.nbr[hits * a.n + i] = j;
             ++hits;
-            density_pair(r2, P, t3, u3);
+            W.pair(r2, P);
         }
     }
     return hits;
@@ -162,7 +175,7 @@ __device__ __forceinline__ u32 density_direct_row(const DevParams& P, const Trav
 template <class C>
 __device__ __forceinline__ u32 density_staged_row(const DevParams& P, const TravArgs& a, BlockSmem<C>& S, u32 i,
                                                   float4 xi, const u32* rpref, u32 seg0, u32 Dy, u32 Dz, u32 selfm,
-                                                  bool act, float& t3, float& u3) {
+                                                  bool act, DensitySum& W) {
     const float2 nx = make_float2(-xi.x, -xi.x), ny = make_float2(-xi.y, -xi.y), nz = make_float2(-xi.z, -xi.z);
     const float lim = -__uint_as_float(__float_as_uint(P.h2) + 1u);   // minus the float after h2
     const float2 nlim = make_float2(lim, lim);
@@ -241,7 +254,7 @@ __device__ __forceinline__ u32 density_staged_row(const DevParams& P, const Trav
                 const float r2 = dist2(xi, make_float4(S.x[m], S.y[m], S.z[m], 0.f));
                 if (listed) a.nbr[slot_idx] = S.j[m];
                 slot_idx += a.n;
-                density_pair(r2, P, t3, u3);
+                W.pair(r2, P);
             } while (w);
         }
     } while (seg < 9u);
@@ -385,7 +398,7 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
                     const u32 i = i0 + (act ? r : 0u);
                     const u64 pk = a.ckey[i];
                     const float4 xi = ro_ld(a.pos + guard(a, i, n));
-                    float t3 = 0.f, u3 = 0.f;
+                    DensitySum W;
                     u32 hits = 0;
                     if (staged) {
                         u32 cx, cy, cz, sc;
@@ -397,12 +410,12 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
                         const u32 s = S.rstart[b][cell], m0 = S.rpref[b][cell];
                         const u32 selfm = i - s < S.rpref[b][cell + 1u] - m0 ? m0 + (i - s) : 0xFFFF0000u;
                         hits = density_staged_row<C>(P, a, S, i, xi, S.rpref[b], cell - ring, G.Dy, G.Dz, selfm,
-                                                     act && in, t3, u3);
+                                                     act && in, W);
                     } else if (act) {
-                        hits = density_direct_row<BATCH>(P, a, i, pk, xi, t3, u3);
+                        hits = density_direct_row<BATCH>(P, a, i, pk, xi, W);
                     }
                     if (act) {
-                        const float res[1] = {__fmaf_rn(2.f, t3, -u3)};
+                        const float res[1] = {W.value()};
                         float resb[1] = {0.f};
                         if (a.nb > 0) density_boundary_row<BATCH>(P, a, xi, G.scene, i, resb);
                         float r_max = 0.f, r_s = 0.f, r_s2 = 0.f;
