@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(CS_THREADS, 1) cluster_sort_kernel(const Clust
         a.st->sort_sel[SORT_DIGITS] = 1u;
         a.st->unit_count = 0;
         a.st->unit_next = 0;
+        a.st->thin_count = 0;
+        a.st->thin_rows = 0;
     }
     for (u32 t = me * CS_THREADS + tid; t < a.table_size; t += blocks * CS_THREADS) a.table[t] = EMPTY_HASH;
     cluster_barrier(cluster, blocks);

@@ -60,6 +60,15 @@ struct BlockCfg<6> {   // 4x4x4 cells
     static constexpr int nt = 288, cap = 2560, words = 12, min_blocks = 3;
 };
 
+// Thin units (up to thin_rows(level) particles) per thread block above which
+// their rows are summed one lane each from global memory, 32 to a warp, instead
+// of unit by unit. A unit costs a block's look-ups of 64 to 216 cells whatever it
+// holds (some 5 us of one of 444 to 1184 resident blocks), a batch of rows one
+// chain of 27 look-ups (about 30 us) that all blocks can share. Step time in us,
+// units / rows (the pass before the blocks): 60 k scattered particles 318 / 110
+// (188), 400 k 4123 / 300 (736), 1 M with 100 k of spray 1533 / 845 (1298); but
+// 2 k scattered 50 / 72, and 20 k at 1.2 a cell (2 k thin units) 72 / 101.
+constexpr u32 THIN_UNITS = 6;
 constexpr int BLOCK_CELLS = 216;   // cells of the largest block with its surrounding layer
 
 template <class C>
@@ -77,6 +86,9 @@ struct BlockSmem {
     u32 rows[2];       // its particles
     u32 next;          // the unit claimed next
     u32 chunk;         // look-up chunks handed out
+    // work items: `thin` thin units (by_rows: batches of their rows), then the
+    // others (here and not in registers, which the row loop needs)
+    u32 items, thin, by_rows;
 };
 
 // Density of row i's boundary particles (cell size h cells, one lane): its
@@ -98,17 +110,27 @@ __device__ __forceinline__ void density_boundary_row(const DevParams& P, const T
         const u32 b0 = t + 32u * w;
         const u32 len = min(32u, e - b0);
         u32 bits = 0;
-#pragma unroll 4
-        for (u32 u = 0; u < len; ++u) {
-            const float4 xb = ro_ld(a.bcx + guard(a, b0 + u, a.bcx_n));
-            bits |= (dist2(xi, xb) <= P.h2 ? 1u : 0u) << u;
+        // four in flight, past the end the last one again (as an unrolled loop the
+        // compiler kept them in flight or not by the code around it: 2 k particles
+        // 62 against 66 us a step)
+        for (u32 u = 0; u < len; u += 4u) {
+            float4 xb[4];
+#pragma unroll
+            for (u32 v = 0; v < 4u; ++v) xb[v] = ro_ld(a.bcx + guard(a, b0 + min(u + v, len - 1u), a.bcx_n));
+#pragma unroll
+            for (u32 v = 0; v < 4u; ++v) bits |= (dist2(xi, xb[v]) <= P.h2 ? 1u : 0u) << (u + v);
         }
+        bits &= FULL >> (32u - len);
 #pragma unroll
         for (u32 q = 0; q < 4; ++q)
             if (w == q) mk[q] = bits;
-        for (; bits; bits &= bits - 1) {
-            const float4 xb = ro_ld(a.bcx + guard(a, b0 + (__ffs(bits) - 1), a.bcx_n));
-            boundary_pair_m<PASS_DENSITY>(resb, H, xb.w, xb, dist2(xi, xb), P);
+        float4 xb = xi;
+        if (bits) xb = ro_ld(a.bcx + guard(a, b0 + (__ffs(bits) - 1), a.bcx_n));
+        while (bits) {   // the next hit is in flight while one is summed
+            const float4 now = xb;
+            bits &= bits - 1;
+            if (bits) xb = ro_ld(a.bcx + guard(a, b0 + (__ffs(bits) - 1), a.bcx_n));
+            boundary_pair_m<PASS_DENSITY>(resb, H, now.w, now, dist2(xi, now), P);
         }
     }
     if (a.bmask != nullptr) a.bmask[i] = make_uint4(mk[0], mk[1], mk[2], mk[3]);
@@ -140,30 +162,45 @@ struct DensitySum {
     __device__ __forceinline__ float value() const { return __fmaf_rn(2.f, t3, -__fmaf_rn(2.f, over, u3)); }
 };
 
-// Row i without staged candidates (a single cell whose 27 cells exceed the
-// capacity): its cells one after the other from global memory, in the same
-// order. Returns the neighbour count.
+// Row i without staged candidates (a thin block, or a single cell whose 27
+// cells exceed the capacity): its cells from global memory, in the same order,
+// three looked up at a time. Returns the neighbour count.
 template <bool BATCH>
 __device__ __forceinline__ u32 density_direct_row(const DevParams& P, const TravArgs& a, u32 i, u64 pk, float4 xi,
                                                   DensitySum& W) {
     u32 ux, uy, uz, scene;
     decode_cell<BATCH>(pk, ux, uy, uz, scene);
     u32 hits = 0;
-    for (u32 q = 0; q < 27u; ++q) {
-        int dx, dy, dz;
-        cell_offset(q, 1, dx, dy, dz);
-        u64 ck;
-        if constexpr (BATCH) ck = pack_cell_batch(scene, ux + dx, uy + dy, uz + dz);
-        else ck = pack_cell(ux + dx, uy + dy, uz + dz);
-        const u32 slot = find_slot<BATCH>(a.fluid.table, a.fluid.tmask, ck);
-        if (slot == EMPTY_CELL) continue;
-        const u32 e = ro_ld(a.fluid.cend + slot);
-        for (u32 j = ro_ld(a.fluid.cstart + slot); j < e; ++j) {
-            const float r2 = dist2(xi, ro_ld(a.pos + guard(a, j, a.n)));
-            if (!(r2 <= P.h2) || j == i) continue;
-            if (hits < a.nbr_width) a.nbr[hits * a.n + i] = j;
-            ++hits;
-            W.pair(r2, P);
+    for (u32 q = 0; q < 9u; ++q) {
+        const u32 x = ux + q / 3u - 1u, y = uy + q % 3u - 1u;
+        u64 ck[3], seen[3];
+        u32 slot[3], s[3], e[3];
+#pragma unroll
+        for (u32 u = 0; u < 3u; ++u) {
+            if constexpr (BATCH) ck[u] = pack_cell_batch(scene, x, y, uz + u - 1u);
+            else ck[u] = pack_cell(x, y, uz + u - 1u);
+            slot[u] = static_cast<u32>(slot_hash<BATCH>(ck[u])) & a.fluid.tmask;
+            seen[u] = ro_ld(a.fluid.table + slot[u]);
+        }
+#pragma unroll
+        for (u32 u = 0; u < 3u; ++u) {
+            if (seen[u] != ck[u])
+                slot[u] = seen[u] == EMPTY_HASH ? EMPTY_CELL : find_slot<BATCH>(a.fluid.table, a.fluid.tmask, ck[u]);
+            s[u] = e[u] = 0u;
+            if (slot[u] != EMPTY_CELL) {
+                s[u] = ro_ld(a.fluid.cstart + slot[u]);
+                e[u] = ro_ld(a.fluid.cend + slot[u]);
+            }
+        }
+#pragma unroll
+        for (u32 u = 0; u < 3u; ++u) {
+            for (u32 j = s[u]; j < e[u]; ++j) {
+                const float r2 = dist2(xi, ro_ld(a.pos + guard(a, j, a.n)));
+                if (!(r2 <= P.h2) || j == i) continue;
+                if (hits < a.nbr_width) a.nbr[hits * a.n + i] = j;
+                ++hits;
+                W.pair(r2, P);
+            }
         }
     }
     return hits;
@@ -324,12 +361,19 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
     const u32 tid = threadIdx.x;
     const u32 lane = tid & 31u;
     const u32 n = a.n;
-    const u32 count = *reinterpret_cast<const volatile u32*>(&a.st->unit_count);
+    const volatile DevState& st = *a.st;
+    if (tid == 0) {
+        const u32 by_rows = st.thin_count > THIN_UNITS * gridDim.x ? 1u : 0u;
+        S.by_rows = by_rows;
+        S.thin = by_rows ? (st.thin_rows + C::nt - 1u) / C::nt : st.thin_count;
+        S.items = S.thin + st.unit_count;
+    }
+    volatile BlockSmem<C>& V = S;
     const u64 unit_mask = block_mask<BATCH>(a.unit_level);
-    // the first claim of every block is its own index
-    if (blockIdx.x >= count) return;
     auto lookup_unit = [&](u32 u, u32 b) {
-        const u32 start = guard(a, a.units[u], n);
+        const u32 thin = V.thin;
+        if (u < thin && V.by_rows) return;
+        const u32 start = guard(a, a.units[u < thin ? n - 1u - u : u - thin], n);
         const u64 id = a.ckey[start] & unit_mask;
         if (tid == 0) {
             S.start[b] = start;
@@ -342,13 +386,15 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
         S.rows[0] = 0u;
     }
     __syncthreads();
-    lookup_unit(blockIdx.x, 0u);
-    for (u32 b = 0;; b ^= 1u) {
+    u32 item = blockIdx.x;   // the first claim of every block is its own index
+    if (item < V.items) lookup_unit(item, 0u);
+    for (u32 b = 0; item < V.items; b ^= 1u) {
         u32 claimed = 0;
         if (tid == 0) claimed = atomicAdd(&a.st->unit_next, 1u) + gridDim.x;
         __syncthreads();   // the unit's look-ups, and the last rows of the one before
+        const bool listed = item < V.thin && V.by_rows;   // rows of thin units
         u32 level = a.unit_level;
-        u32 i0 = S.start[b];
+        u32 i0 = listed ? item * C::nt : S.start[b];
         u64 id = S.id[b];
         for (;;) {
             const BlockGrid<BATCH> G(id, level);
@@ -356,7 +402,7 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
             // exclusive prefix of the counts
             if (tid < 32u) {
                 u32 run = 0;
-                for (u32 base = 0; base < ncell; base += 32u) {
+                for (u32 base = 0; base < ncell && !listed; base += 32u) {
                     const u32 q = base + lane;
                     const u32 c = q < ncell ? S.rpref[b][q] : 0u;
                     const u32 incl = warp_incl_scan(c);
@@ -372,9 +418,9 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
             }
             __syncthreads();
             const u32 M = S.rpref[b][ncell];
-            const u32 rows = min(S.rows[b], n - i0);
+            const u32 rows = listed ? min(static_cast<u32>(C::nt), st.thin_rows - i0) : min(S.rows[b], n - i0);
             const bool split = M > static_cast<u32>(C::cap) && level > 0u;   // too dense: smaller blocks
-            const bool staged = M <= static_cast<u32>(C::cap);
+            const bool staged = M <= static_cast<u32>(C::cap) && !listed;
             if (staged) {
                 // eight lanes per cell: a cell's particles are contiguous
                 for (u32 q = tid >> 3; q < ncell; q += C::nt / 8) {
@@ -395,14 +441,15 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
                 for (u32 r0 = tid & ~31u; r0 < rows; r0 += C::nt) {
                     const u32 r = r0 + lane;
                     const bool act = r < rows;
-                    const u32 i = i0 + (act ? r : 0u);
+                    u32 i = i0 + (act ? r : 0u);
+                    if (listed) i = guard(a, a.units[n + i], n);
                     const u64 pk = a.ckey[i];
+                    u32 cx, cy, cz, scene;
+                    decode_cell<BATCH>(pk, cx, cy, cz, scene);
                     const float4 xi = ro_ld(a.pos + guard(a, i, n));
                     DensitySum W;
                     u32 hits = 0;
                     if (staged) {
-                        u32 cx, cy, cz, sc;
-                        decode_cell<BATCH>(pk, cx, cy, cz, sc);
                         cx -= G.ox; cy -= G.oy; cz -= G.oz;   // 1 .. D - 2 per axis
                         const bool in = cx - 1u < G.Dx - 2u && cy - 1u < G.Dy - 2u && cz - 1u < G.Dz - 2u;
                         const u32 ring = (G.Dy + 1u) * G.Dz + 1u;   // from the first of the 27 cells to their middle
@@ -417,13 +464,13 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
                     if (act) {
                         const float res[1] = {W.value()};
                         float resb[1] = {0.f};
-                        if (a.nb > 0) density_boundary_row<BATCH>(P, a, xi, G.scene, i, resb);
+                        if (a.nb > 0) density_boundary_row<BATCH>(P, a, xi, scene, i, resb);
                         float r_max = 0.f, r_s = 0.f, r_s2 = 0.f;
                         finish_row<PASS_DENSITY, BATCH>(P, a, i, res, resb, hits <= a.nbr_width ? hits : NBR_SPILL,
-                                                        G.scene, 0.f, 0.f, r_max, r_s, r_s2);
+                                                        scene, 0.f, 0.f, r_max, r_s, r_s2);
                     }
                 }
-                if (level == a.unit_level) break;
+                if (listed || level == a.unit_level) break;
                 i0 += rows;
                 if (rows == 0u || i0 >= n || (a.ckey[i0] & unit_mask) != S.id[b]) break;   // the same for every thread
             } else {
@@ -440,9 +487,8 @@ __device__ __forceinline__ void density_units(const DevParams& P, const TravArgs
             density_lookup<C, BATCH>(a, S, b, id, level);
             __syncthreads();
         }
-        const u32 next = S.next;
-        if (next >= count) return;
-        lookup_unit(next, b ^ 1u);
+        item = S.next;
+        if (item < V.items) lookup_unit(item, b ^ 1u);
     }
 }
 

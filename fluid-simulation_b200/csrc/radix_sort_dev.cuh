@@ -143,6 +143,8 @@ __device__ __forceinline__ void sort_plan_block(u32 n, u32* WCSPH_SORT_RESTRICT 
         st->first_active = first;
         st->unit_count = 0;   // listed again by the reorder
         st->unit_next = 0;
+        st->thin_count = 0;
+        st->thin_rows = 0;
         st->sort_narrow = narrow_keys(st) ? 1u : 0u;
         for (int d = 0; d < 3; ++d) st->cell_lo[d] = st->cell_hi[d] = 0;   // for the next sort
     }

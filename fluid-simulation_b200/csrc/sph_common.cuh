@@ -316,10 +316,12 @@ struct DevState {
     u32 sort_tile_counter[8];
     u32 first_active;           // first active pass (generates the iota values)
     u32 sort_narrow;            // the compressed keys are u32 words
-    // density units (blocks of cells): listed by the reorder, claimed by the
-    // density pass; both reset by the sort plan
+    // density units (blocks of cells), thin ones apart and also as rows: listed
+    // by the reorder, claimed by the density pass; all reset with the sort
     u32 unit_count;
     u32 unit_next;
+    u32 thin_count;
+    u32 thin_rows;
     // cell-coordinate bounds of the particles of the current sort (0 is always
     // included; reset to 0 by the sort plan): they choose the compressed keys
     int cell_lo[3];

@@ -1675,16 +1675,29 @@ __device__ __forceinline__ void reorder_cell_item(const float4* WCSPH_RESTRICT p
     // changes and ends (non-inclusive) at the next change.
     const bool first = valid && (i == 0 || pk != prev);
     const bool last = valid && (i == n - 1 || pk != next);
-    if (units) {   // list the blocks of 2^unit_level cells that start here, in any order
+    if (units) {
+        // list the blocks of 2^unit_level cells that start here, in any order:
+        // from entry 0 up, thin ones (that also end in this warp) from n - 1 down,
+        // and the rows of these from n up
         const u64 bm = block_mask<BATCH>(unit_level);
         const bool opens = valid && (i == 0 || ((pk ^ prev) & bm) != 0ull);
-        const u32 starts = __ballot_sync(FULL, opens);
-        if (starts) {
-            u32 at = 0;
-            if (lane == 0) at = atomicAdd(&st_err->unit_count, static_cast<u32>(__popc(starts)));
-            at = __shfl_sync(FULL, at, 0);
-            if (opens) units[at + __popc(starts & ((1u << lane) - 1u))] = i;
-        }
+        const bool closes = valid && (i == n - 1 || ((pk ^ next) & bm) != 0ull);
+        const u32 open = __ballot_sync(FULL, opens) & (FULL >> (31u - lane));   // the last of them opened i's block
+        const u32 close = __ballot_sync(FULL, closes) & (FULL << lane);         // the first of them closes it
+        const bool thin = valid && open != 0u && close != 0u &&
+                          static_cast<u32>(__ffs(static_cast<int>(close)) - 32 + __clz(static_cast<int>(open))) <
+                              thin_rows(unit_level);
+        const u32 thick_here = __ballot_sync(FULL, opens && !thin), thin_here = __ballot_sync(FULL, opens && thin);
+        const u32 rows_here = __ballot_sync(FULL, thin);
+        u32 at = 0;
+        if (lane == 0 && thick_here) at = atomicAdd(&st_err->unit_count, static_cast<u32>(__popc(thick_here)));
+        if (lane == 1 && thin_here) at = atomicAdd(&st_err->thin_count, static_cast<u32>(__popc(thin_here)));
+        if (lane == 2 && thin_here) at = atomicAdd(&st_err->thin_rows, static_cast<u32>(__popc(rows_here)));
+        const u32 thick_at = __shfl_sync(FULL, at, 0), thin_at = n - 1u - __shfl_sync(FULL, at, 1),
+                  row_at = n + __shfl_sync(FULL, at, 2);
+        const u32 lt = (1u << lane) - 1u;
+        if (opens) units[thin ? thin_at - __popc(thin_here & lt) : thick_at + __popc(thick_here & lt)] = i;
+        if (thin) units[row_at + __popc(rows_here & lt)] = i;
     }
     u32 slot = EMPTY_CELL;
     if (first) {

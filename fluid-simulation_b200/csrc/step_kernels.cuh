@@ -92,8 +92,9 @@ struct TravArgs {
     u32 matrix_valid;         // neighbour export: the mask buffer holds the last density pass's matrix
     u32 chunk;                // sorted particles per warp chunk: 8, 16 or 32
     // density units: first sorted particle of each Morton-aligned block of
-    // 2^unit_level cells (count in st->unit_count; nullptr: the density pass
-    // takes chunks of cells)
+    // 2^unit_level cells (2 n entries: st->unit_count blocks from the first on,
+    // st->thin_count thin ones from entry n - 1 down, their st->thin_rows rows
+    // from entry n on); nullptr: the density pass takes chunks of cells
     const u32* units;
     u32 unit_level;
     // neighbour lists (nullptr: the force and surface passes walk the bit matrix)
@@ -167,6 +168,14 @@ inline int list_warps(int kind, u32 n) { return n < LIST_SMALL ? 2 : (kind == 1 
 // 393 k with walls 136 / 119 / 128, 0.7 M settled 246 / 257 / 258, 1 M
 // 254 / 222 / 204, 4 M 1092 / 939 / 831.
 inline u32 unit_level(u32 n) { return n < (1u << 18) ? 3u : (n < (1u << 19) ? 5u : 6u); }
+
+// Particles up to which a unit counts as thin (density_units sums the rows of
+// many thin units without staging): one warp of the reorder sees such a unit
+// whole, and its rows cost less than a unit's look-ups. Step time in us at 4 / 8
+// / 16 rows in 2x2x2 cells: 60 k particles at 4 a unit 150 / 131 / 131, 100 k
+// 229 / 195 / 189; at 8 / 16 / 24 rows in 4x4x2 cells: 400 k at 13 a unit
+// 656 / 500 / 480.
+__host__ __device__ constexpr u32 thin_rows(u32 level) { return level == 3u ? 8u : 16u; }
 
 void launch_pass(int kind, const DevParams& P, const TravArgs& a, cudaStream_t stream, int warps_per_block,
                  bool batch = false);
