@@ -36,12 +36,15 @@ __device__ __forceinline__ u32 ld_volatile(const u32* p) { return *reinterpret_c
 // Work counters of the traversal phases (after the barrier words): warps take
 // CLAIM chunks at a time, so that no block idles at a barrier while others
 // still hold a long queue. Block 0 clears them with the sort plan of each step.
+// List groups are 32 rows: a warp takes no more at a time than leaves some for
+// every warp (four regardless, and at 37 k particles 288 of 3552 warps had all
+// the work).
 enum : u32 { WORK_DENSITY = 2, WORK_FORCE = 3, WORK_SURFACE = 4, BARRIER_WORDS = 5 };
 constexpr u32 CLAIM = 4;
 
-__device__ __forceinline__ u32 claim(u32* ctr) {
+__device__ __forceinline__ u32 claim(u32* ctr, u32 size = CLAIM) {
     u32 v = 0;
-    if ((threadIdx.x & 31u) == 0) v = atomicAdd(ctr, CLAIM);
+    if ((threadIdx.x & 31u) == 0) v = atomicAdd(ctr, size);
     return __shfl_sync(0xffffffffu, v, 0);
 }
 
@@ -166,10 +169,11 @@ __global__ void __launch_bounds__(PTHREADS, PERSISTENT_BLOCKS) persistent_ensemb
         }
         if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;
         const u32 ngroups = (n + LIST_ROWS - 1) / LIST_ROWS;
+        const u32 take = min(CLAIM, max(1u, ngroups / (gridDim.x * PWARPS)));
         if (UNITS || a.nbr) {
-            for (u32 g0 = claim(ps.barrier + WORK_FORCE); g0 < ngroups; g0 = claim(ps.barrier + WORK_FORCE))
-                for (u32 g = g0; g < min(g0 + CLAIM, ngroups); ++g)
-                    list_rows<PASS_FORCE, true, 2>(P, a, g * LIST_ROWS, min(LIST_ROWS, n - g * LIST_ROWS), 0.f, 0.f, rm, rs, rs2);
+            for (u32 g0 = claim(ps.barrier + WORK_FORCE, take); g0 < ngroups; g0 = claim(ps.barrier + WORK_FORCE, take))
+                for (u32 g = g0; g < min(g0 + take, ngroups); ++g)
+                    list_rows<PASS_FORCE, true, 2, 1>(P, a, g * LIST_ROWS, min(LIST_ROWS, n - g * LIST_ROWS), 0.f, 0.f, rm, rs, rs2);
         } else {
             const WarpView<PASS_FORCE> S = warp_view<PASS_FORCE>(a, smem, warp);
             for (u32 c0 = claim(ps.barrier + WORK_FORCE); c0 < nchunks; c0 = claim(ps.barrier + WORK_FORCE))
@@ -179,9 +183,9 @@ __global__ void __launch_bounds__(PTHREADS, PERSISTENT_BLOCKS) persistent_ensemb
         if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;
         const float dt = cfl_time_step(a, P);   // fixed step: the bounds alone decide
         if (UNITS || a.nbr) {
-            for (u32 g0 = claim(ps.barrier + WORK_SURFACE); g0 < ngroups; g0 = claim(ps.barrier + WORK_SURFACE))
-                for (u32 g = g0; g < min(g0 + CLAIM, ngroups); ++g)
-                    list_rows<PASS_SURFACE, true, 2>(P, a, g * LIST_ROWS, min(LIST_ROWS, n - g * LIST_ROWS), dt, np_dt, rm, rs, rs2);
+            for (u32 g0 = claim(ps.barrier + WORK_SURFACE, take); g0 < ngroups; g0 = claim(ps.barrier + WORK_SURFACE, take))
+                for (u32 g = g0; g < min(g0 + take, ngroups); ++g)
+                    list_rows<PASS_SURFACE, true, 2, 1>(P, a, g * LIST_ROWS, min(LIST_ROWS, n - g * LIST_ROWS), dt, np_dt, rm, rs, rs2);
         } else {
             const WarpView<PASS_SURFACE> S = warp_view<PASS_SURFACE>(a, smem, warp);
             for (u32 c0 = claim(ps.barrier + WORK_SURFACE); c0 < nchunks; c0 = claim(ps.barrier + WORK_SURFACE))

@@ -1110,6 +1110,60 @@ __device__ __forceinline__ void spill_row(const DevParams& P, const TravArgs& a,
     }
 }
 
+// The fluid sums of up to G rows of one cell (particles i[0 .. m)) without
+// their lists: lane q walks neighbour cells q, q + 32, ... of the cell (its hash
+// probe and particles), testing every candidate against h^2 for each row; a
+// row's lane partials are then added in a fixed butterfly order, so a row's sums
+// do not depend on its group. Leaves the sums on every lane.
+// Bound by latency (a look-up, then a record load per candidate): the rows of a
+// group share both, and the next record is in flight. (spill_row, for one row,
+// keeps the registers of the kernels that have none to spare.)
+template <int KIND, bool BATCH, int G>
+__device__ __forceinline__ void spill_rows(const DevParams& P, const TravArgs& a, const u32 (&i)[G], u32 m, u64 pk,
+                                           float (&v)[G][KindCfg<KIND>::nf]) {
+    constexpr int NF = KindCfg<KIND>::nf;
+    const u32 lane = lane_id();
+    u32 ux, uy, uz, scene;
+    decode_cell<BATCH>(pk, ux, uy, uz, scene);
+    const int R = a.range;
+    const u32 D = static_cast<u32>(2 * R + 1);
+    const u32 ncell = D * D * D;
+    HomeData H[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        H[g] = load_home<KIND>(a, i[g]);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[g][f] = 0.f;
+    }
+    for (u32 q = lane; q < ncell; q += 32) {
+        int dx, dy, dz;
+        cell_offset(q, R, dx, dy, dz);
+        u64 ck;
+        if constexpr (BATCH) ck = pack_cell_batch(scene, ux + dx, uy + dy, uz + dz);
+        else ck = pack_cell(ux + dx, uy + dy, uz + dz);
+        const u32 slot = find_slot<BATCH>(a.fluid.table, a.fluid.tmask, ck);
+        if (slot == EMPTY_CELL) continue;
+        const u32 e = ro_ld(a.fluid.cend + slot);
+        u32 j = ro_ld(a.fluid.cstart + slot);
+        Nbr next;
+        if (j < e) next = fetch_j<KIND>(a, j);
+        for (; j < e; ++j) {
+            const Nbr d = next;
+            if (j + 1u < e) next = fetch_j<KIND>(a, j + 1u);
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const float r2 = dist2(H[g].x, d.x);
+                if (r2 <= P.h2 && j != i[g] && static_cast<u32>(g) < m) fluid_pair<KIND>(v[g], H[g], d, r2, P, a);
+            }
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+            for (int o = 16; o > 0; o >>= 1) v[g][f] += __shfl_xor_sync(FULL, v[g][f], o);
+}
+
 // Boundary sums of one row (particle i, home data H): the 3x3x3 boundary
 // cells around its own cell in x, y, z nesting order, as for_boundary_neighbors
 // (common.cuh:153-178) visits them, one particle after the other.
@@ -1183,27 +1237,63 @@ __device__ __forceinline__ void boundary_row(const DevParams& P, const TravArgs&
 // row k's list in order (the reference's per-particle order), so a row's
 // sums do not depend on which particles share its warp.
 // DEPTH: neighbours summed together, with the next DEPTH in flight.
-template <int KIND, bool BATCH, int DEPTH>
+// G: spilled rows of one cell summed together (spill_rows). SHARE warps take the
+// same rows: the first those with lists, and each its share of the spilled ones.
+template <int KIND, bool BATCH, int DEPTH, int G, int SHARE = 1>
 __device__ __forceinline__ void list_rows(const DevParams& P, const TravArgs& a, u32 i0, u32 nh, float dt,
-                                          float np_dt, float& red_max, float& red_speed, float& red_speed2) {
+                                          float np_dt, float& red_max, float& red_speed, float& red_speed2,
+                                          u32 part = 0u) {
     using C = KindCfg<KIND>;
     constexpr int NF = C::nf;
     constexpr int NFB = C::nfb;
     const u32 lane = lane_id();
-    const bool act = lane < nh;
-    const u32 i = i0 + (act ? lane : 0u);
-    const u32 cnt = act ? ro_ld(a.nbr_cnt + i) : 0u;
-    const bool spill = act && cnt > a.nbr_width;
+    const bool row = lane < nh;
+    const u32 i = i0 + (row ? lane : 0u);
+    const u32 cnt = row ? ro_ld(a.nbr_cnt + i) : 0u;
+    const bool spill = row && cnt > a.nbr_width;
+    u32 sp = __ballot_sync(FULL, spill);
+    bool act = row;
+    if constexpr (SHARE > 1) {
+        const u32 rank = __popc(sp & ((1u << lane) - 1u)) / G;
+        act = row && (spill ? rank % SHARE == part : part == 0u);
+        sp = __ballot_sync(FULL, spill && act);
+        if (part != 0u && sp == 0u) return;
+    }
     float res[NF], resb[NFB];
 #pragma unroll
     for (int f = 0; f < NF; ++f) res[f] = 0.f;
-    for (u32 sp = __ballot_sync(FULL, spill); sp; sp &= sp - 1) {
-        const u32 f = __ffs(sp) - 1;
-        float t[NF];
-        spill_row<KIND, BATCH>(P, a, i0 + f, t);
-        if (lane == f) {
+    if constexpr (G == 1) {
+        for (; sp; sp &= sp - 1) {
+            const u32 f = __ffs(sp) - 1;
+            float t[NF];
+            spill_row<KIND, BATCH>(P, a, i0 + f, t);
+            if (lane == f) {
 #pragma unroll
-            for (int g = 0; g < NF; ++g) res[g] = t[g];
+                for (int g = 0; g < NF; ++g) res[g] = t[g];
+            }
+        }
+    } else {
+        while (sp) {
+            // the next spilled rows of one cell (a cell's rows follow one another)
+            const u32 first = __ffs(static_cast<int>(sp)) - 1;
+            const u64 cell = a.ckey[i0 + first];
+            u32 left = __ballot_sync(FULL, spill && a.ckey[i] == cell) & sp;
+            u32 at[G], id[G], m = 0;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                at[g] = left ? __ffs(static_cast<int>(left)) - 1 : first;
+                id[g] = i0 + at[g];
+                m += left ? 1u : 0u;
+                sp &= left ? ~(1u << at[g]) : FULL;
+                left &= left - 1u;
+            }
+            float t[G][NF];
+            spill_rows<KIND, BATCH, G>(P, a, id, m, cell, t);
+#pragma unroll
+            for (int g = G - 1; g >= 0; --g)   // the group's first row last: the places of absent rows name it too
+                if (lane == at[g])
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) res[f] = t[g][f];
         }
     }
 #pragma unroll

@@ -61,15 +61,19 @@ density_block_kernel(const DevParams P, const TravArgs a) {
 // Smaller scenes leave the SMs a few warps each, so three at a time are summed
 // with 128 registers to spare: force / surface 27 / 27 -> 20 / 16 us at 33 k
 // particles with walls, 55 / 55 -> 27 / 25 at 79 k (half of that by full warps:
-// these scenes took 8 rows per warp before).
+// these scenes took 8 rows per warp before). Rows without usable lists are
+// summed two at a time there (`spilled`; four would take 121 registers: the 79 k
+// step 128 -> 143 us): all rows of 79 k particles with 32 list slots 540 -> 459
+// us a step, 513 with 8 rows per warp.
 template <int KIND, bool SMALL>
 struct ListCfg {
     static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : 48);
     static constexpr int depth = SMALL ? 3 : (KIND == PASS_FORCE ? 2 : 1);
+    static constexpr int spilled = SMALL ? 2 : 1;
 };
 
 // Force / surface pass over the neighbour lists written by the density pass.
-template <int KIND, int WPB, bool BATCH, bool SMALL>
+template <int KIND, int WPB, bool BATCH, bool SMALL, int SHARE>
 __global__ void __launch_bounds__(WPB * 32, ListCfg<KIND, SMALL>::min_warps / WPB)
 list_pass_kernel(const DevParams P, const TravArgs a) {
     if (a.st->error_flags & ERR_LOOKBACK_TIMEOUT) return;   // no sorted state this step (reorder skipped)
@@ -83,10 +87,11 @@ list_pass_kernel(const DevParams P, const TravArgs a) {
         np_dt = a.delta < a.np_max_dt ? a.delta : a.np_max_dt;
     }
     float red_max = 0.f, red_speed = 0.f, red_speed2 = 0.f;
-    const u32 base = (blockIdx.x * WPB + warp) * LIST_ROWS;
+    const u32 gw = blockIdx.x * WPB + warp;
+    const u32 base = gw / SHARE * LIST_ROWS;
     if (base < a.n)
-        list_rows<KIND, BATCH, ListCfg<KIND, SMALL>::depth>(P, a, base, min(LIST_ROWS, a.n - base), dt, np_dt, red_max,
-                                                            red_speed, red_speed2);
+        list_rows<KIND, BATCH, ListCfg<KIND, SMALL>::depth, ListCfg<KIND, SMALL>::spilled, SHARE>(
+            P, a, base, min(LIST_ROWS, a.n - base), dt, np_dt, red_max, red_speed, red_speed2, gw % SHARE);
     if constexpr (KIND == PASS_SURFACE) surface_reduce<WPB>(a, dt, np_dt, red_max, red_speed, red_speed2);
 }
 
@@ -197,8 +202,10 @@ static void launch_wpb(const DevParams& P, const TravArgs& a, cudaStream_t strea
     // per-warp candidate staging sized by the bit-matrix capacity 32 * mask_words
     if constexpr (KIND == PASS_FORCE || KIND == PASS_SURFACE) {
         if (a.nbr) {   // the list kernels use no shared memory (all of it serves as L1)
-            if (a.n < LIST_SMALL) list_pass_kernel<KIND, WPB, BATCH, true><<<grid, WPB * 32, 0, stream>>>(P, a);
-            else list_pass_kernel<KIND, WPB, BATCH, false><<<grid, WPB * 32, 0, stream>>>(P, a);
+            const dim3 block(WPB * 32);
+            if (list_share(a.n) > 1u) list_pass_kernel<KIND, WPB, BATCH, true, LIST_SHARE><<<grid, block, 0, stream>>>(P, a);
+            else if (a.n < LIST_SMALL) list_pass_kernel<KIND, WPB, BATCH, true, 1><<<grid, block, 0, stream>>>(P, a);
+            else list_pass_kernel<KIND, WPB, BATCH, false, 1><<<grid, block, 0, stream>>>(P, a);
             return;
         }
     }
@@ -238,7 +245,8 @@ static void launch_density_blocks(const DevParams& P, const TravArgs& a, cudaStr
 template <int KIND, bool BATCH>
 static void launch_kind(const DevParams& P, const TravArgs& a, cudaStream_t stream, int wpb) {
     const bool listed = (KIND == PASS_FORCE || KIND == PASS_SURFACE) && a.nbr != nullptr;
-    const u32 grid = pass_grid(a.n, wpb, listed ? LIST_ROWS : a.chunk);
+    const u32 groups = (a.n + LIST_ROWS - 1) / LIST_ROWS;   // each of list_share warps
+    const u32 grid = listed ? pass_grid(groups * list_share(a.n), wpb, 1u) : pass_grid(a.n, wpb, a.chunk);
     if (grid == 0) return;
     if constexpr (KIND == PASS_DENSITY) {
         if (a.units) {

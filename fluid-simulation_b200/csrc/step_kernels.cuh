@@ -159,6 +159,14 @@ void launch_reorder_cells(const float4* pos_in, const float4* vel_in, const u32*
 // against 55 / 55 before it, 135 k 34 / 34 against 30 / 28, 198 k 40 / 50
 // against 42 / 40, 250 k 44-48 / 50-56 against 44-46 / 52-58.
 constexpr u32 LIST_SMALL = 1u << 17;
+// Warps that take the same 32 rows of the list passes: in the smallest scenes,
+// whose warps leave the SMs idle, four, so that rows without usable lists, which
+// a warp sums one or two at a time, are shared out (2 k particles with 32 list
+// slots: 253 us a step by one warp, 117 by four). Where the SMs are full the
+// extra warps cost more than any such row: two per 32 rows take the 33 k step
+// from 93 to 100 us, the 79 k step from 128 to 151.
+constexpr int LIST_SHARE = 4;
+inline u32 list_share(u32 n) { return n < (1u << 14) ? LIST_SHARE : 1u; }
 inline int list_warps(int kind, u32 n) { return n < LIST_SMALL ? 2 : (kind == 1 ? 4 : 8); }
 
 // Cells per density unit (BlockCfg), as a power of two. Larger units look up
@@ -183,7 +191,7 @@ void launch_pass(int kind, const DevParams& P, const TravArgs& a, cudaStream_t s
 u32 pass_grid(u32 n, int warps_per_block, u32 chunk);
 // Upper bound of the warps of any traversal launch over n particles (chunk >= 8,
 // at most 8 warps per block): sizes the surface pass's reduction buffers.
-inline u32 pass_max_warps(u32 n) { return (n + 7u) / 8u + 8u; }
+inline u32 pass_max_warps(u32 n) { return (n + 31u) / 32u * 4u + 8u; }
 
 // CFL max |v|^2 of a velocity array into st->vmax2_bits[st->parity].
 void launch_init_cfl(const float4* vel, u32 n, DevState* st, cudaStream_t stream);
