@@ -394,4 +394,9 @@ int wcsph_test_stall_sort(int enable) {
     return WCSPH_OK;
 }
 
+int wcsph_test_large_sort(int enable) {
+    wcsph::set_large_sort_test(enable != 0);
+    return WCSPH_OK;
+}
+
 }  // extern "C"

@@ -332,7 +332,7 @@ cudaError_t launch_ipt(const ClusterSortArgs& a, cudaStream_t stream, bool* laun
 
 cudaError_t enqueue_cluster_sort(const ClusterSortArgs& a, cudaStream_t stream, bool* launched) {
     *launched = false;
-    if (a.n == 0 || a.n > CLUSTER_SORT_MAX || sort_stall_test()) return cudaSuccess;
+    if (a.n == 0 || a.n > CLUSTER_SORT_MAX || sort_stall_test() || large_sort_test()) return cudaSuccess;
     if (!a.pos) return launch_ipt<SORT_KEYS>(a, stream, launched);
     if (a.scene) return launch_ipt<SORT_BATCH>(a, stream, launched);
     return launch_ipt<SORT_SCENE>(a, stream, launched);

@@ -42,7 +42,8 @@ struct ClusterSortArgs {
 
 // Enqueues the sort on `stream`. *launched = false, and nothing is enqueued,
 // where it does not apply: too many keys, a device on which the cluster does not
-// fit, or the look-back stall test hook is on (that tests the onesweep's waits).
+// fit, or a test hook of the onesweep is on (its waits, or its results at sizes
+// that the cluster takes).
 cudaError_t enqueue_cluster_sort(const ClusterSortArgs& a, cudaStream_t stream, bool* launched);
 
 }  // namespace wcsph

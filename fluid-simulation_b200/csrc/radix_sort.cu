@@ -9,10 +9,13 @@ namespace wcsph {
 
 namespace {
 std::atomic<bool> g_sort_stall_test{false};
+thread_local bool t_large_sort_test = false;
 }
 
 void set_sort_stall_test(bool on) { g_sort_stall_test.store(on); }
 bool sort_stall_test() { return g_sort_stall_test.load(); }
+void set_large_sort_test(bool on) { t_large_sort_test = on; }
+bool large_sort_test() { return t_large_sort_test; }
 
 
 __global__ void keys_hist_kernel(const float4* __restrict__ pos, u32 n, float cs,

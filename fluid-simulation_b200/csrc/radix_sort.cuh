@@ -95,5 +95,9 @@ cudaError_t enqueue_sort_passes(const SortBuffers& b, u32 n, DevState* st, cudaS
 // look-back flags and wait at most LB_SPIN_LIMIT_STALLED polls.
 void set_sort_stall_test(bool on);
 bool sort_stall_test();
+// Test hook of the calling thread: while on, the sorts it enqueues take the
+// onesweep where the cluster sort would run.
+void set_large_sort_test(bool on);
+bool large_sort_test();
 
 }  // namespace wcsph

@@ -202,6 +202,7 @@ def load_library(path: str | os.PathLike | None = None) -> C.CDLL:
         "wcsph_rollout_backward": (C.c_int, [vp, f, f, f]),
         "wcsph_sort_keys_static": (C.c_int, [vp, C.c_uint32, vp, vp]),
         "wcsph_test_stall_sort": (C.c_int, [C.c_int]),
+        "wcsph_test_large_sort": (C.c_int, [C.c_int]),
         "wcsph_camera_look": (None, [f, C.c_float, C.c_float, C.c_uint32, C.c_uint32, C.POINTER(Camera)]),
         "wcsph_default_render_opts": (None, [C.POINTER(RenderOpts)]),
         "wcsph_render": (C.c_int, [vp, C.POINTER(Camera), C.POINTER(RenderOpts), vp, f]),
@@ -437,6 +438,19 @@ class stall_sort:
 
     def __exit__(self, *exc):
         load_library().wcsph_test_stall_sort(0)
+        return False
+
+
+class large_sort:
+    """Test hook (wcsph_test_large_sort): inside the block, sorts enqueued by this
+    thread take the path of large scenes at any size."""
+
+    def __enter__(self):
+        load_library().wcsph_test_large_sort(1)
+        return self
+
+    def __exit__(self, *exc):
+        load_library().wcsph_test_large_sort(0)
         return False
 
 

@@ -390,18 +390,22 @@ int wcsph_render(wcsph_ctx* ctx, const wcsph_camera* cam, const wcsph_render_opt
  * stable sort permutation of the n device-resident 64-bit keys (perm[i] = index
  * of the key of rank i, equal keys in input order): the same permutation the
  * step's sort produces (WCSPH_FIELD_PERMUTATION for WCSPH_FIELD_MORTON_KEYS).
- * keys is only read. Nothing is allocated: the scratch is a device array of the
- * library image, about 1.8 MiB, that every GPU loading the library holds until
- * the process exits.
+ * keys is only read. Nothing is allocated: one launch of a thread-block cluster
+ * sorts in shared memory. On a device where that cluster does not fit (and under
+ * the test hooks below) a fallback sorts in a device array of the library image,
+ * about 1.8 MiB, that every GPU loading the library holds until the process exits.
  *   - n above WCSPH_STATIC_SORT_MAX_KEYS returns WCSPH_ERR_INVALID_ARGUMENT
  *     (text via wcsph_last_error(NULL)); n == 0 does nothing.
  *   - The work is enqueued on `stream` (a cudaStream_t; NULL = the default
  *     stream) of the current device and the call returns without waiting.
+ *   - The cluster sort keeps nothing between calls: they may overlap on the GPU
+ *     (other streams, other host threads) and be captured from the first on.
+ * Of the fallback alone:
  *   - The first call on a device looks up the scratch's device address (set-up
  *     done once per device); make that first call before any stream capture.
  *   - Every call on a device shares the one scratch: calls whose work overlaps
- *     on the GPU (other streams, other host threads) race and corrupt each
- *     other's results. Order them on one stream or synchronise between them.
+ *     on the GPU race and corrupt each other's results. Order them on one
+ *     stream or synchronise between them.
  *   - The sort's waits between its tiles are bounded (about a second). If one
  *     runs out, the call cannot tell the host without waiting for the GPU, so
  *     it marks its output instead: every perm entry is then
@@ -414,7 +418,7 @@ int wcsph_render(wcsph_ctx* ctx, const wcsph_camera* cam, const wcsph_render_opt
 #define WCSPH_STATIC_SORT_FAILED 0xFFFFFFFFu
 int wcsph_sort_keys_static(const uint64_t* keys, uint32_t n, uint32_t* perm, void* stream);
 
-/* ---- error-path test hook ---------------------------------------------------
+/* ---- test hooks ---------------------------------------------------------------
  * No counterpart in the reference. While `enable` is non-zero, every radix sort
  * enqueued afterwards (the step's, the boundary set-up's, the batch's and
  * wcsph_sort_keys_static) withholds its first tile's look-back flags and bounds
@@ -425,6 +429,13 @@ int wcsph_sort_keys_static(const uint64_t* keys, uint32_t n, uint32_t* perm, voi
  * in a CUDA graph keep the setting they were captured with. Nothing faults or
  * hangs: it exists only to test these error paths. Returns WCSPH_OK.          */
 int wcsph_test_stall_sort(int enable);
+
+/* While `enable` is non-zero, sorts that the calling thread enqueues (the
+ * step's, the batch's per-stage ones, wcsph_sort_keys_static) take the path of
+ * large scenes, and of devices on which the cluster does not fit, at any size:
+ * the same permutations. Steps already captured keep the path they were captured
+ * with. It exists only to test that path. Returns WCSPH_OK.                   */
+int wcsph_test_large_sort(int enable);
 
 #ifdef __cplusplus
 }
