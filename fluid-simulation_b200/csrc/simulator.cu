@@ -361,6 +361,7 @@ bool CUDASPHSimulator::enqueue_small_sort() {
     c.table_size = table_size_;
     bool launched = false;
     WCSPH_CUDA(enqueue_cluster_sort(c, stream_, &launched));
+    cluster_sorted_ = launched;
     return launched;
 }
 
@@ -420,9 +421,9 @@ void CUDASPHSimulator::enqueue_step(float delta) {
 }
 
 int CUDASPHSimulator::launches_per_step() const {
-    // small scenes: cluster sort, else keys_bounds + compressed_keys_hist + sort_plan + 8 onesweep;
-    // then reorder_cells and the three passes
-    return (n_ <= CLUSTER_SORT_MAX ? 1 : 2 + 1 + SORT_DIGITS) + 1 + 3;
+    // cluster sort, or keys_bounds + compressed_keys_hist + sort_plan + 8 onesweep (as the last
+    // step enqueued them; before any, as the size says); then reorder_cells and the three passes
+    return (cluster_sorted_.value_or(n_ <= CLUSTER_SORT_MAX) ? 1 : 2 + 1 + SORT_DIGITS) + 1 + 3;
 }
 
 void CUDASPHSimulator::invalidate_graph() {

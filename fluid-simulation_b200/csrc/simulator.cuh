@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -277,6 +278,7 @@ private:
     cudaGraphExec_t graph_exec_ = nullptr;
     float graph_delta_ = 0.f;
     bool graph_valid_ = false;
+    std::optional<bool> cluster_sorted_;   // how the last step enqueued was sorted
     bool stepped_since_state_ = false;
     bool was_tuning_step_ = false;
 

@@ -83,3 +83,18 @@ def test_staged_batch_matches_the_cluster_sort():
     with wcsph.large_sort():
         got = run()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_launches_per_step_are_those_of_the_path():
+    pos = np.ones((3000, 4), np.float32)
+    pos[:, :3] = np.random.default_rng(0).random((3000, 3))
+    p = wcsph.default_params(particle_radius=0.02, max_time_step=1e-4, cfl_factor=0.0)
+    for hook, want in ((None, 5), (wcsph.large_sort, 15)):
+        with wcsph.CUDASPHSimulator(p, pos, wcsph.box((0, 0, 0), (1, 1, 1))) as sim:
+            if hook:
+                with hook():
+                    sim.update(1e-4)
+            else:
+                sim.update(1e-4)
+            sim.synchronize()
+            assert sim.launches_per_step() == want
