@@ -5,6 +5,7 @@
 #include <atomic>
 #include <climits>
 
+#include "simulator.cuh"
 #include "step_device.cuh"
 
 namespace wcsph {
@@ -226,20 +227,21 @@ static void launch_density_blocks(const DevParams& P, const TravArgs& a, cudaStr
     constexpr int kMaxDevices = 64;
     static std::atomic<u32> resident[kMaxDevices];   // resident blocks of the device, 0 = not yet asked
     int dev = 0;
-    cudaGetDevice(&dev);
+    WCSPH_CUDA(cudaGetDevice(&dev));
     u32 blocks = dev < kMaxDevices ? resident[dev].load() : 0u;
     // on every call: the attribute belongs to the current context
-    cudaFuncSetAttribute(density_block_kernel<LEVEL, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(sizeof(BlockSmem<C>)));
+    WCSPH_CUDA(cudaFuncSetAttribute(density_block_kernel<LEVEL, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(sizeof(BlockSmem<C>))));
     if (blocks == 0) {
         int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, density_block_kernel<LEVEL, BATCH>, C::nt,
-                                                      sizeof(BlockSmem<C>));
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        WCSPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, density_block_kernel<LEVEL, BATCH>, C::nt,
+                                                                 sizeof(BlockSmem<C>)));
+        WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         blocks = static_cast<u32>(std::max(per_sm, 1) * std::max(sms, 1));
         if (dev < kMaxDevices) resident[dev].store(blocks);
     }
     density_block_kernel<LEVEL, BATCH><<<std::min(blocks, a.n), C::nt, sizeof(BlockSmem<C>), stream>>>(P, a);
+    WCSPH_CUDA(cudaGetLastError());
 }
 
 template <int KIND, bool BATCH>
