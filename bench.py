@@ -18,6 +18,7 @@ sources into oracle/_ref by oracle/build_ref.py) on the same workload.
 from __future__ import annotations
 
 import argparse
+import ctypes as C
 import json
 import os
 import statistics
@@ -98,63 +99,76 @@ def measured_limits(workload: str, n: int, kernel: str):
 
 
 class ClockSampler:
-    """nvidia-smi samples of SM clock and throttle reasons during the timed region."""
+    """SM clock and throttle reasons during the timed region, read through NVML by
+    a thread (a region of twenty steps takes 13 ms, and nvidia-smi does not deliver
+    a sample within that). Reads only."""
 
-    FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
-              "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
-              "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
+    REASONS = {0x8: "hw_slowdown", 0x40: "hw_thermal_slowdown", 0x20: "sw_thermal_slowdown", 0x4: "sw_power_cap"}
+    SM_CLOCK = 1
 
-    def __init__(self, device: int):
-        self.device = device
-        self.rows = []
-        self.proc = None
+    def __init__(self, device: int, nvml=None):
+        self.rows = []   # (SM MHz, reason bits)
+        self.sm_max = None
+        self.nvml = None
+        self.stop = threading.Event()
+        try:
+            lib = nvml if nvml is not None else C.CDLL("libnvidia-ml.so.1")
+            handle = C.c_void_p()
+            if lib.nvmlInit_v2() == 0 and self._find(lib, device, handle) == 0:
+                self.nvml, self.handle = lib, handle
+                mx = C.c_uint()
+                if lib.nvmlDeviceGetMaxClockInfo(handle, self.SM_CLOCK, C.byref(mx)) == 0:
+                    self.sm_max = float(mx.value)
+        except (OSError, AttributeError):
+            pass
+
+    @staticmethod
+    def _find(lib, device, handle):
+        """NVML's handle of CUDA device `device` (CUDA_VISIBLE_DEVICES may renumber them)."""
+        try:
+            import torch
+
+            uuid = f"GPU-{torch.cuda.get_device_properties(device).uuid}".encode()
+            if lib.nvmlDeviceGetHandleByUUID(uuid, C.byref(handle)) == 0:
+                return 0
+        except Exception:
+            pass
+        return lib.nvmlDeviceGetHandleByIndex_v2(C.c_uint(device), C.byref(handle))
+
+    def _read(self):
+        clock, bits = C.c_uint(), C.c_ulonglong()
+        while not self.stop.is_set():
+            if (self.nvml.nvmlDeviceGetClockInfo(self.handle, self.SM_CLOCK, C.byref(clock)) == 0
+                    and self.nvml.nvmlDeviceGetCurrentClocksThrottleReasons(self.handle, C.byref(bits)) == 0):
+                self.rows.append((float(clock.value), int(bits.value)))
+            self.stop.wait(0.0005)
 
     def __enter__(self):
-        try:
-            self.proc = subprocess.Popen(
-                ["nvidia-smi", f"--id={self.device}", f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits",
-                 "-lms", "20"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+        if self.nvml is not None:
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
-        except Exception:
-            self.proc = None
         return self
 
     def wait_first(self, busy, limit_s: float = 3.0):
-        """Runs `busy` (keeps the clocks up) until the sampler delivers, then
-        drops those samples: the timed region starts with the sampler running
-        (a step takes well under a millisecond, the sampler's start a hundred)."""
+        """Runs `busy` (keeps the clocks up) until the sampler delivers, then drops
+        those samples: the timed region starts with the sampler running."""
         t0 = time.perf_counter()
-        while self.proc is not None and not self.rows and time.perf_counter() - t0 < limit_s:
+        while self.nvml is not None and not self.rows and time.perf_counter() - t0 < limit_s:
             busy()
         self.rows.clear()
 
-    def _read(self):
-        for line in self.proc.stdout:
-            self.rows.append([x.strip() for x in line.split(",")])
-
     def __exit__(self, *a):
-        if self.proc is not None:
-            self.proc.terminate()
-            try:
-                self.proc.wait(timeout=5)
-            except Exception:
-                self.proc.kill()
+        self.stop.set()
+        if self.nvml is not None:
+            self.t.join(timeout=5)
 
     def summary(self):
-        if not self.rows:
-            return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["unsampled"]}
-        sm = [float(r[1]) for r in self.rows if len(r) > 8 and r[1].replace(".", "").isdigit()]
-        mx = [float(r[2]) for r in self.rows if len(r) > 8 and r[2].replace(".", "").isdigit()]
-        names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        reasons = set()
-        for r in self.rows:
-            if len(r) > 8:
-                for k, name in enumerate(names):
-                    if r[5 + k].lower().startswith("active"):
-                        reasons.add(name)
-        return {"sm_mhz": statistics.median(sm) if sm else None, "sm_max_mhz": max(mx) if mx else None,
-                "reasons": sorted(reasons), "samples": len(self.rows)}
+        rows = list(self.rows)
+        if not rows:
+            return {"sm_mhz": None, "sm_max_mhz": self.sm_max, "reasons": ["unsampled"]}
+        reasons = {name for _, bits in rows for bit, name in self.REASONS.items() if bits & bit}
+        return {"sm_mhz": statistics.median(c for c, _ in rows), "sm_max_mhz": self.sm_max,
+                "reasons": sorted(reasons), "samples": len(rows)}
 
 
 def dist_setup():
