@@ -191,6 +191,20 @@ void CUDASPHSimulator::allocate() {
     WCSPH_CUDA(cudaMemcpyAsync(box_dev_.ptr, &box_host_, sizeof(DevBox), cudaMemcpyHostToDevice, stream_));
 }
 
+u32 CUDASPHSimulator::list_width(const StepConfig& c) const {
+    // list slots are addressed with 32-bit indices: very large scenes get
+    // fewer slots (rows that do not fit are recomputed), or none below 8
+    uint64_t width = static_cast<uint64_t>(c.nbr_width);
+    if (n_ > 0) width = std::min<uint64_t>(width, ((1ull << 32) - 1) / n_);
+    return width >= 8 ? static_cast<u32>(width) : 0u;
+}
+
+bool CUDASPHSimulator::uses_units(const StepConfig& c) const {
+    wcsph_params p = params_;
+    p.cell_size_mult = c.cell_size_mult;
+    return list_width(c) > 0 && make_dev_params(p).range == 1;
+}
+
 void CUDASPHSimulator::ensure_tables() {
     const u32 t = fluid_table_size();
     if (t != table_size_) {
@@ -205,11 +219,7 @@ void CUDASPHSimulator::ensure_tables() {
         mask_.alloc(words);
         WCSPH_CUDA(cudaMemsetAsync(mask_.ptr, 0, mask_.bytes(), stream_));
     }
-    // list slots are addressed with 32-bit indices: very large scenes get
-    // fewer slots (rows that do not fit are recomputed), or none below 8
-    uint64_t width = static_cast<uint64_t>(cfg_.nbr_width);
-    if (n_ > 0) width = std::min<uint64_t>(width, ((1ull << 32) - 1) / n_);
-    nbr_width_ = width >= 8 ? static_cast<u32>(width) : 0u;
+    nbr_width_ = list_width(cfg_);
     const size_t slots = static_cast<size_t>(n_) * nbr_width_;
     if (nbr_.count != slots) {
         nbr_.alloc(slots);

@@ -168,6 +168,8 @@ public:
 
     // tuning
     const StepConfig& config() const { return cfg_; }
+    // Whether a step under c takes its density pass over blocks of cells.
+    bool uses_units(const StepConfig& c) const;
     void apply_config(const StepConfig& c);
     void set_tuning(int searcher, float budget, const char* frozen_json);
     bool was_tuning_step() const { return was_tuning_step_; }
@@ -214,6 +216,7 @@ private:
     // The density pass works on blocks of cells (density_blocks.cuh) where the
     // lists are on and the neighbourhood is one cell deep.
     bool use_units() const { return nbr_width_ > 0 && dp_.range == 1; }
+    u32 list_width(const StepConfig& c) const;
     // Unit list: the sort's second key buffer, free once the sort is done.
     u32* unit_buf() { return reinterpret_cast<u32*>(keys_[1].ptr); }
 

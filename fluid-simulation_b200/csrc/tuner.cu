@@ -131,6 +131,22 @@ bool config_allowed(const StepConfig& c) {
 }
 }  // namespace
 
+// Where the density pass takes blocks of cells, its block size, the bit-matrix
+// words and the particles per warp change nothing in a step: such configurations
+// carry one value of each. (45 equal ones apiece otherwise; a search would time
+// the same launches again and choose among them by noise.)
+StepConfig Tuner::normalised(StepConfig c) const {
+    const StepConfig base;
+    if (sim_->uses_units(c)) {
+        c.warps_density = base.warps_density;
+        c.mask_words = base.mask_words;
+        c.chunk = base.chunk;
+    } else if (c.chunk == 0) {
+        c.chunk = static_cast<int>(effective_chunk(c, sim_->get_fluid_particles()));
+    }
+    return c;
+}
+
 Tuner::Tuner(CUDASPHSimulator* sim) : sim_(sim) {
     for (int wd : kWarps)
         for (int wf : kWarps)
@@ -143,7 +159,10 @@ Tuner::Tuner(CUDASPHSimulator* sim) : sim_(sim) {
                                 c.warps_density = wd; c.warps_force = wf; c.warps_surface = ws;
                                 c.mask_words = mw; c.chunk = ch;
                                 c.cell_size_mult = static_cast<float>(cm); c.table_size_mult = tm;
-                                if (config_allowed(c)) space_.push_back(c);
+                                if (!config_allowed(c)) continue;
+                                const bool lead = wd == kWarps[0] && mw == kMaskWords[0] && ch == kChunk[0];
+                                if (!sim->uses_units(c)) space_.push_back(c);
+                                else if (lead) space_.push_back(normalised(c));
                             }
     visited_.assign(space_.size(), 0);
     best_cfg_ = sim->config();
@@ -233,6 +252,8 @@ int Tuner::next_candidate() {
         }
         default: shift(c.table_size_mult, kTableMult, 6); break;
         }
+        c = normalised(c);
+        if (c == cur) continue;   // a parameter at its end, or one that changes nothing here
         for (int k = 0; k < n; ++k)
             if (space_[k] == c) return k;
     }

@@ -3,10 +3,11 @@
 // space step_tuner.cuh:79-121,326-357, TuningScheduler
 // tuning_scheduler.h:12-26, load_config_json config_loader.cpp:8-54).
 //
-// Search space (StepConfig): warps per block of the three cell passes,
-// neighbour-bitmask words (list capacity vs on-the-fly rescan), cell-size
-// multiplier and hash-table multiplier, under the reference's constraint
-// TABLE_SIZE_MULT >= uint64(1 / CELL_SIZE_MULT^3) (step_tuner.cuh:94-99).
+// Search space (StepConfig): warps per block of the force and surface passes,
+// cell-size multiplier and hash-table multiplier, under the reference's constraint
+// TABLE_SIZE_MULT >= uint64(1 / CELL_SIZE_MULT^3) (step_tuner.cuh:94-99); where the
+// density pass takes cells one by one (two cells a radius), also its warps per
+// block, the neighbour-bitmask words and the particles per warp.
 // Searchers: MCMC (Metropolis walk over neighbouring configurations), random
 // (uniform without replacement) and full (deterministic enumeration).
 // Each tuning iteration times one real step with CUDA events.
@@ -47,6 +48,7 @@ public:
 
 private:
     int next_candidate();
+    StepConfig normalised(StepConfig c) const;
     CUDASPHSimulator* sim_;
     std::vector<StepConfig> space_;
     std::vector<char> visited_;
