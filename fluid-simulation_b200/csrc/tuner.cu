@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <fstream>
+#include <iterator>
 #include <sstream>
 
 namespace wcsph {
@@ -148,21 +149,28 @@ StepConfig Tuner::normalised(StepConfig c) const {
 }
 
 Tuner::Tuner(CUDASPHSimulator* sim) : sim_(sim) {
+    bool units[std::size(kCellMult)];   // by cell size
+    for (size_t k = 0; k < std::size(kCellMult); ++k) {
+        StepConfig c;
+        c.cell_size_mult = static_cast<float>(kCellMult[k]);
+        units[k] = sim->uses_units(c);
+    }
     for (int wd : kWarps)
         for (int wf : kWarps)
             for (int ws : kWarps)
                 for (int mw : kMaskWords)
                     for (int ch : kChunk)
-                        for (double cm : kCellMult)
+                        for (size_t cm = 0; cm < std::size(kCellMult); ++cm)
                             for (uint32_t tm : kTableMult) {
                                 StepConfig c;
-                                c.warps_density = wd; c.warps_force = wf; c.warps_surface = ws;
-                                c.mask_words = mw; c.chunk = ch;
-                                c.cell_size_mult = static_cast<float>(cm); c.table_size_mult = tm;
-                                if (!config_allowed(c)) continue;
-                                const bool lead = wd == kWarps[0] && mw == kMaskWords[0] && ch == kChunk[0];
-                                if (!sim->uses_units(c)) space_.push_back(c);
-                                else if (lead) space_.push_back(normalised(c));
+                                c.warps_force = wf; c.warps_surface = ws;
+                                c.cell_size_mult = static_cast<float>(kCellMult[cm]); c.table_size_mult = tm;
+                                if (!units[cm]) {
+                                    c.warps_density = wd; c.mask_words = mw; c.chunk = ch;
+                                } else if (wd != kWarps[0] || mw != kMaskWords[0] || ch != kChunk[0]) {
+                                    continue;
+                                }
+                                if (config_allowed(c)) space_.push_back(c);
                             }
     visited_.assign(space_.size(), 0);
     best_cfg_ = sim->config();
