@@ -58,7 +58,9 @@ density_block_kernel(const DevParams P, const TravArgs a) {
 // 141 -> 121 us, 4 M 497 -> 430 (28 warps 126 / 461, 40 warps spill: 166 / 629,
 // three at a time 136 / 505). The surface pass keeps one at a time, all the
 // warps that fit and 8-warp blocks: 1 M 139 us, 4 M 474 (two at a time at 32
-// warps 143 / 516; 2-warp blocks 141 / 502).
+// warps 143 / 516; 2-warp blocks 141 / 502); the batched one, which looks its
+// scene up, would spill at 40 registers and takes 48 (12 and 100 scenes 256 / 1090
+// -> 252 / 1088 us a step).
 // Smaller scenes leave the SMs a few warps each, so three at a time are summed
 // with 128 registers to spare: force / surface 27 / 27 -> 20 / 16 us at 33 k
 // particles with walls, 55 / 55 -> 27 / 25 at 79 k (half of that by full warps:
@@ -66,16 +68,16 @@ density_block_kernel(const DevParams P, const TravArgs a) {
 // summed two at a time there (`spilled`; four would take 121 registers: the 79 k
 // step 128 -> 143 us): all rows of 79 k particles with 32 list slots 540 -> 459
 // us a step, 513 with 8 rows per warp.
-template <int KIND, bool SMALL>
+template <int KIND, bool SMALL, bool BATCH = false>
 struct ListCfg {
-    static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : 48);
+    static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : (BATCH ? 40 : 48));
     static constexpr int depth = SMALL ? 3 : (KIND == PASS_FORCE ? 2 : 1);
     static constexpr int spilled = SMALL ? 2 : 1;
 };
 
 // Force / surface pass over the neighbour lists written by the density pass.
 template <int KIND, int WPB, bool BATCH, bool SMALL, int SHARE>
-__global__ void __launch_bounds__(WPB * 32, ListCfg<KIND, SMALL>::min_warps / WPB)
+__global__ void __launch_bounds__(WPB * 32, ListCfg<KIND, SMALL, BATCH>::min_warps / WPB)
 list_pass_kernel(const DevParams P, const TravArgs a) {
     if (a.st->error_flags & ERR_LOOKBACK_TIMEOUT) return;   // no sorted state this step (reorder skipped)
     const u32 lane = lane_id();
