@@ -143,9 +143,9 @@ __global__ void __launch_bounds__(PTHREADS, PERSISTENT_BLOCKS) persistent_ensemb
                 __syncthreads();
                 const u32 tile = s_tile;
                 if (tile >= ps.tiles) break;
-                sortdev::onesweep_tile<u64, false>(n, p, ps.keys[0], ps.keys[1], ps.keys[2], ps.vals[1], ps.vals[2], ps.offsets,
-                                       ps.lookback, ps.tiles, st, ps.spin_limit, 0u, tile,
-                                            *reinterpret_cast<sortdev::TileSmem*>(smem));
+                sortdev::onesweep_tile<u64, false>(n, p, ps.keys[0], ps.keys[1], ps.keys[2], ps.vals[1], ps.vals[2],
+                                                   ps.offsets, ps.lookback, ps.tiles, st, ps.spin_limit, 0u, tile,
+                                                   *reinterpret_cast<sortdev::TileSmem*>(smem));
                 __syncthreads();
             }
             if (!grid_barrier(ps.barrier, st, ps.barrier_limit)) return;

@@ -22,17 +22,17 @@
 // within a few hits, and no partial sums cross lanes: a row's sum runs over its
 // neighbours in the reference's order whatever the block size.
 //
-// What bounds it (1 M particles, 4x4x4 cells): instruction issue (141 M warp
-// instructions, 61 % of the cycles issue) and the shared-memory data pipe
-// (75 % busy: a 128-bit load costs three wavefronts for a warp's four or five
-// cells, a walked hit four loads of four). Of 208 us, look-ups took about 35
-// (latency; 203 since warps that are done look up for the next unit), staging
-// 18, the tests 85, the walk 61, the epilogue 18. The pass it replaced gave a
-// warp the two cells of an x-pair (36 looked-up cells and 18 staged candidates
-// per row, where a row here pays for 3.4), split their hits over the lanes and
-// wrote the lists one scattered word at a time: 349 M warp instructions, 460 us
-// (4 M particles 2055 -> 830 us, 0.7 M settled 434 -> 258, 33 k with walls
-// 51 -> 30).
+// What bounds it (1 M particles, 4x4x4 cells, ten steps into a run): instruction
+// issue (166 M warp instructions, 64 % of the cycles issue) and the shared-memory
+// data pipe (76 % busy: a 128-bit load costs three wavefronts for a warp's four or
+// five cells, a walked hit four loads of four). Of the lattice's 213 us, before
+// the sums carried their errors, look-ups took 34 (latency; 9 less since warps
+// that are done look up for the next unit), staging 14, the tests 85, the walk 57,
+// the epilogue 23. The pass it replaced gave a warp the two cells of an x-pair (36
+// looked-up cells and 18 staged candidates per row, where a row here pays for
+// 3.4), split their hits over the lanes and wrote the lists one scattered word at
+// a time: 349 M warp instructions, 460 us (4 M particles 2055 -> 830 us, 0.7 M
+// settled 434 -> 258, 33 k with walls 51 -> 30).
 #pragma once
 
 namespace wcsph {

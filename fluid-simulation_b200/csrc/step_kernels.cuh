@@ -173,8 +173,9 @@ inline int list_warps(int kind, u32 n) { return n < LIST_SMALL ? 2 : (kind == 1 
 // and stage fewer cells per row (8, 4.5 and 3.4 candidates a row), smaller
 // ones give more thread blocks and a shorter last wave. Density pass in us at
 // levels 3 / 5 / 6: 33 k particles with walls 30 / 35 / 48, 79 k 53 / 65 / 80,
-// 393 k with walls 136 / 119 / 128, 0.7 M settled 246 / 257 / 258, 1 M
-// 254 / 222 / 204, 4 M 1092 / 939 / 831.
+// 393 k with walls 136 / 119 / 128, 1 M 254 / 222 / 204, 4 M 1092 / 939 / 831 (all
+// lattices). The count alone decides; a settled fluid, whose cells are uneven,
+// gains less from large units: 0.7 M settled 246 / 257 / 258.
 inline u32 unit_level(u32 n) { return n < (1u << 18) ? 3u : (n < (1u << 19) ? 5u : 6u); }
 
 // Particles up to which a unit counts as thin (density_units sums the rows of
