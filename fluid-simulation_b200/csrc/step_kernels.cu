@@ -68,7 +68,7 @@ density_block_kernel(const DevParams P, const TravArgs a) {
 // summed two at a time there (`spilled`; four would take 121 registers: the 79 k
 // step 128 -> 143 us): all rows of 79 k particles with 32 list slots 540 -> 459
 // us a step, 513 with 8 rows per warp.
-template <int KIND, bool SMALL, bool BATCH = false>
+template <int KIND, bool SMALL, bool BATCH>
 struct ListCfg {
     static constexpr int min_warps = SMALL ? 16 : (KIND == PASS_FORCE ? 36 : (BATCH ? 40 : 48));
     static constexpr int depth = SMALL ? 3 : (KIND == PASS_FORCE ? 2 : 1);
@@ -93,7 +93,7 @@ list_pass_kernel(const DevParams P, const TravArgs a) {
     const u32 gw = blockIdx.x * WPB + warp;
     const u32 base = gw / SHARE * LIST_ROWS;
     if (base < a.n)
-        list_rows<KIND, BATCH, ListCfg<KIND, SMALL>::depth, ListCfg<KIND, SMALL>::spilled, SHARE>(
+        list_rows<KIND, BATCH, ListCfg<KIND, SMALL, BATCH>::depth, ListCfg<KIND, SMALL, BATCH>::spilled, SHARE>(
             P, a, base, min(LIST_ROWS, a.n - base), dt, np_dt, red_max, red_speed, red_speed2, gw % SHARE);
     if constexpr (KIND == PASS_SURFACE) surface_reduce<WPB>(a, dt, np_dt, red_max, red_speed, red_speed2);
 }
