@@ -197,7 +197,7 @@ __device__ __forceinline__ u32 density_direct_row(const DevParams& P, const Trav
             // four in flight, past the end the last one again (one at a time 120
             // particles a cell took 2.26 ms a step, so 1.56)
             for (u32 j0 = s[u]; j0 < e[u]; j0 += 4u) {
-                float r2[4u];
+                float r2[4];
 #pragma unroll
                 for (u32 v = 0; v < 4u; ++v)
                     r2[v] = dist2(xi, ro_ld(a.pos + guard(a, min(j0 + v, e[u] - 1u), a.n)));
